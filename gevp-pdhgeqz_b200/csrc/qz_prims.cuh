@@ -261,20 +261,28 @@ QZ_HD void shift_column(double h11, double h21, double h12, double h22, double h
 // Eigenvalues of a 2x2 pencil (A, B), B upper triangular (b10 = 0), as
 // the coefficients of the real quadratic c2*l^2 - c1*l + c0 with
 //   c2 = b00*b11, c1 = a00*b11 + a11*b00 - a10*b01, c0 = a00*a11 - a01*a10.
-QZ_HD void pencil2_poly(double a00, double a10, double a01, double a11,
-                        double b00, double b01, double b11,
-                        double& c2, double& c1, double& c0) {
-  double sa = dmax(dmax(fabs(a00), fabs(a10)), dmax(fabs(a01), fabs(a11)));
-  double sb = dmax(dmax(fabs(b00), fabs(b01)), fabs(b11));
+// pencil2_scaled gives them for A / sa, B / sb (sa, sb: the largest entries),
+// where nothing can overflow or underflow: l = (sa/sb) l'.
+QZ_HD void pencil2_scaled(double a00, double a10, double a01, double a11, double b00, double b01, double b11,
+                          double& c2, double& c1, double& c0, double& sa, double& sb) {
+  sa = dmax(dmax(fabs(a00), fabs(a10)), dmax(fabs(a01), fabs(a11)));
+  sb = dmax(dmax(fabs(b00), fabs(b01)), fabs(b11));
   if (sa == 0.0) sa = 1.0;
   if (sb == 0.0) sb = 1.0;
   a00 /= sa; a10 /= sa; a01 /= sa; a11 /= sa;
   b00 /= sb; b01 /= sb; b11 /= sb;
-  // lambda scales by sa/sb: c2*l^2 - c1*l + c0 with l = (sa/sb) l'
-  double k = sa / sb;
   c2 = b00 * b11;
-  c1 = (a00 * b11 + a11 * b00 - a10 * b01) * k;
-  c0 = (a00 * a11 - a01 * a10) * k * k;
+  c1 = a00 * b11 + a11 * b00 - a10 * b01;
+  c0 = a00 * a11 - a01 * a10;
+}
+QZ_HD void pencil2_poly(double a00, double a10, double a01, double a11,
+                        double b00, double b01, double b11,
+                        double& c2, double& c1, double& c0) {
+  double sa, sb;
+  pencil2_scaled(a00, a10, a01, a11, b00, b01, b11, c2, c1, c0, sa, sb);
+  const double k = sa / sb;
+  c1 = c1 * k;
+  c0 = c0 * k * k;
 }
 
 // Result of standardising a 2x2 pencil.
@@ -316,8 +324,9 @@ QZ_HD void std2x2(const double* A, const double* B, Std2& o) {
     csl = c; snl = s;
   }
   o.negrow0 = 0; o.negrow1 = 0;
-  double c2, c1, c0;
-  pencil2_poly(a[0], a[1], a[2], a[3], b[0], b[2], b[3], c2, c1, c0);
+  // the characteristic polynomial of A / sa, B / sb
+  double c2, c1, c0, sa, sb;
+  pencil2_scaled(a[0], a[1], a[2], a[3], b[0], b[2], b[3], c2, c1, c0, sa, sb);
   double disc = c1 * c1 - 4.0 * c2 * c0;
   bool cplx = (a[1] != 0.0) && (disc < 0.0) && (c2 != 0.0);
   double rc, rs;  // row rotation (composed later)
@@ -339,13 +348,8 @@ QZ_HD void std2x2(const double* A, const double* B, Std2& o) {
         double mm = dmax(fabs(al), fabs(be));
         al /= mm; be /= mm;
       }
-      double sa = dmax(dmax(fabs(a[0]), fabs(a[1])), dmax(fabs(a[2]), fabs(a[3])));
-      double sb = dmax(dmax(fabs(b[0]), fabs(b[2])), fabs(b[3]));
-      if (sa == 0.0) sa = 1.0;
-      if (sb == 0.0) sb = 1.0;
-      // M = be*A - al*B is singular; (al, be) are in true units.  Divide
-      // the two terms by their natural sizes before forming M.
-      double ka = be / sa, kb = al / sa;
+      // M = be*A/sa - al*B/sb is singular
+      double ka = be / sa, kb = al / sb;
       double m00 = ka * a[0] - kb * b[0], m01 = ka * a[2] - kb * b[2];
       double m10 = ka * a[1],             m11 = ka * a[3] - kb * b[3];
       double n0 = fabs(m00) + fabs(m01), n1 = fabs(m10) + fabs(m11);
