@@ -662,7 +662,7 @@ int b200qz_set_param(b200qz_ctx* c, const char* name, double value) {
   else if (k == "aed_limit") { P.aed_limit = v < 0 ? -1 : v; }
   else if (k == "upd_persist") { if (v != 0 && v != 1) return -3; P.upd_persist = v; }
   else if (k == "split") { if (v != 0 && v != 7 && v != 8) return -3; P.split = v; }
-  else if (k == "aed_threads") { if (v != 32 && v != 64 && v != 128) return -3; P.aed_threads = v; }
+  else if (k == "aed_threads") { if (v != 32 && v != 64 && v != 128 && v != 256) return -3; P.aed_threads = v; }
   else if (k == "aed_swap_fail") { if (v != 0 && v != 1) return -3; P.aed_swap_fail = v; }
   else if (k == "aed_ms") { if (v != 0 && v != 1) return -3; P.aed_ms = v; }
   else if (k == "hr_win") { if (v < 2 || v > qz::kHrMaxWin) return -3; c->hr_win = v; }
@@ -774,7 +774,10 @@ int b200qz_aed_window(b200qz_ctx* c, double* h, double* t, int ld, int ktop, int
   tol.smlnum = DBL_MIN * ((double)nh / DBL_EPSILON);
   tol.htol = std::max(DBL_MIN, DBL_EPSILON * std::sqrt(c->hnorms[0]));
   tol.ttol = std::max(DBL_MIN, DBL_EPSILON * std::sqrt(c->hnorms[1]));
-  launch_aed(c->stream, h, t, ld, ktop, kwtop, nw, tol, qw, zw, shifts, c->dinfo + 4, c->gscratch);
+  // windows in shared memory as the solver runs them, larger ones with the
+  // multishift window QZ
+  launch_aed(c->stream, h, t, ld, ktop, kwtop, nw, tol, qw, zw, shifts, c->dinfo + 4, c->gscratch, nullptr, 0,
+             kRoleThreads, 0, nw > kWinSmemMax ? 1 : 0);
   QZ_CK(cudaMemcpyAsync(c->hinfo + 4, c->dinfo + 4, 3 * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   QZ_CK(cudaStreamSynchronize(c->stream));
   QZ_CK(cudaGetLastError());

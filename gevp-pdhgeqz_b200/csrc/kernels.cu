@@ -14,12 +14,16 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #define QZ_DEFINE_UPDATE_KERNELS
-#include "qz_window.cuh"
+#include "qz_roles.cuh"
 #include "update.cuh"
 #include "kernels.h"
 
 namespace qz {
+
+static_assert(kWinSmemMax <= kRoleMax, "windows of the role-per-warp kernel");
 
 // Executor of the CTA-level algorithms.  With kWarp the CTA is one warp and
 // the barrier is __syncwarp (also a shared-memory fence for the warp).
@@ -65,7 +69,10 @@ __global__ void __launch_bounds__(kThreads) k_aed_win(double* H, double* T, int6
                                                          unsigned long long* ts, int nskip, int swapfail, int ms) {
   extern __shared__ double smem[];
   const int n = nw;
-  const bool in_smem = n <= kWinSmemMax;
+  // the role-per-warp variant takes shared-memory windows only (known at
+  // compile time, so that its accesses are shared-memory instructions)
+  constexpr bool kRoles = kThreads == kRoleThreads;
+  const bool in_smem = kRoles || n <= kWinSmemMax;
   // odd leading dimension in shared memory: row accesses hit distinct banks
   const int lw = in_smem ? smem_ld(n) : n;
   double* Hs;
@@ -86,11 +93,13 @@ __global__ void __launch_bounds__(kThreads) k_aed_win(double* H, double* T, int6
     Zs = Zw;
     sd = smem;
   }
-  // sd: 64 doubles of swap/spike scalars, 4n of spike vectors, the
-  // multishift window QZ's scratch, then the sweep pipeline's buffer
-  int* si = (int*)(sd + 64 + 4 * n + kMsScratch + kPipeDoubles);
+  // sd: 64 doubles of swap/spike scalars, 4n of spike vectors, then the
+  // role buffer, or the multishift window QZ's scratch and the sweep
+  // pipeline's buffer
+  double* const scr = sd + 64 + 4 * n;
+  int* si = (int*)(scr + (kRoles ? kRoleDoubles : kMsScratch + kPipeDoubles));
   DevExecT<kThreads == 32> x{(int)threadIdx.x, kThreads, si, sd, ts};
-  if (kThreads >= 64) x.pipe = (PipeBuf*)(sd + 64 + 4 * n + kMsScratch);
+  if (kThreads >= 64 && !kRoles) x.pipe = (PipeBuf*)(scr + kMsScratch);
   for (int idx = threadIdx.x; idx < n * n; idx += blockDim.x) {
     int i = idx % n, j = idx / n;
     Hs[i + j * lw] = G(H, ld, kwtop + i, kwtop + j);
@@ -109,7 +118,15 @@ __global__ void __launch_bounds__(kThreads) k_aed_win(double* H, double* T, int6
   w.wantq = true;
   w.wantz = true;
   w.tol = tol;
-  cta_aed(x, w, s, shifts, shifts + n, shifts + 2 * n, maxit, nskip, swapfail != 0, ms ? sd + 64 + 4 * n : nullptr);
+  if constexpr (kRoles) {
+    x.stamp(0);
+    const int qz = cta_role_qz(x, w, maxit, (RoleBuf*)scr);
+    if (qz == 0) cta_std_all(x, w, sd + 64);
+    cta_aed_deflate(x, w, s, shifts, shifts + n, shifts + 2 * n, qz, nskip, swapfail != 0,
+                    [&](int m) { return cta_role_hessred(x, w, m, (RoleBuf*)scr); });
+  } else {
+    cta_aed(x, w, s, shifts, shifts + n, shifts + 2 * n, maxit, nskip, swapfail != 0, ms ? scr : nullptr);
+  }
   __syncthreads();
   const int m = si[8], st = si[9], tr = si[10];
   if (st == 0 && tr) {
@@ -396,7 +413,7 @@ __global__ void k_scale_pow2(double* A, int64_t ld, int n, int e) {
 // ---------------------------------------------------------------------------
 size_t aed_smem_bytes(int nw) {
   size_t d = (nw <= kWinSmemMax) ? (size_t)4 * nw * smem_ld(nw) : 0;
-  d += 64 + 4 * (size_t)nw + kMsScratch + kPipeDoubles;
+  d += 64 + 4 * (size_t)nw + std::max(kMsScratch + kPipeDoubles, kRoleDoubles);
   return d * sizeof(double) + kSi * sizeof(int);
 }
 size_t chase_smem_bytes(int wk) {
@@ -427,6 +444,9 @@ cudaError_t kernels_init() {
   e = cudaFuncSetAttribute(k_aed_win<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)aed_smem_bytes(kWinSmemMax));
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(k_aed_win<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)aed_smem_bytes(kWinSmemMax));
+  if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(k_aed_win<kRoleThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)aed_smem_bytes(kWinSmemMax));
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(k_chase_win, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)chase_smem_bytes(kWinSmemMax));
   if (e != cudaSuccess) return e;
@@ -459,7 +479,12 @@ void launch_aed(cudaStream_t st, double* H, double* T, int64_t ld, int ktop, int
                 double* Qw, double* Zw, double* shifts, int* info, double* gscratch, unsigned long long* ts, int nskip,
                 int threads, int swapfail, int ms) {
   const size_t sm = aed_smem_bytes(nw);
-  if (threads <= 32)
+  // a role per warp for windows in shared memory; windows in global memory
+  // and the multishift window QZ run on 128 threads
+  if (threads >= kRoleThreads && nw <= kWinSmemMax && !ms)
+    k_aed_win<kRoleThreads><<<1, kRoleThreads, sm, st>>>(H, T, ld, ktop, kwtop, nw, tol, Qw, Zw, shifts, info, gscratch,
+                                                         30 * nw, ts, nskip, swapfail, ms);
+  else if (threads <= 32)
     k_aed_win<32><<<1, 32, sm, st>>>(H, T, ld, ktop, kwtop, nw, tol, Qw, Zw, shifts, info, gscratch, 30 * nw, ts, nskip,
                                      swapfail, ms);
   else if (threads <= 64)

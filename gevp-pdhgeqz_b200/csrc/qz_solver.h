@@ -35,7 +35,8 @@ struct SolveParams {
                          // -1: whole window for n >= 6000, else 4)
   int max_wave = 8;      // chains chased concurrently (one CTA each)
   int stall_limit = 300; // iterations without deflation before giving up
-  int aed_threads = 128; // threads of the AED / endgame window kernel (32: one warp)
+  int aed_threads = 256; // threads of the AED / endgame window kernel (256: a role
+                         // per warp; 32: one warp)
   int split = 0;         // 7 or 8: off-diagonal updates through that many INT8
                          // Ozaki slices on the tensor cores (windows up to 80)
   int upd_persist = 1;   // 1: persistent, prefetching DMMA update kernels

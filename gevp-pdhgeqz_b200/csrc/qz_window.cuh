@@ -310,13 +310,13 @@ QZ_HD void cta_hessred(X& x, WinState& w, int m) {
   }
 }
 
-template <class X>
-QZ_HD void cta_aed(X& x, WinState& w, double s, double* sr, double* si_, double* sb, int maxit, int nskip = 0,
-                   bool swapfail = false, double* msscr = nullptr) {
-  const bool ms = msscr != nullptr;
+// The part after the window QZ, whose status is info (0: w is in generalized
+// Schur form with standardised blocks).  hessred(m) re-reduces the leading
+// m x m block; false: it failed, and the window with it.
+template <class X, class HR>
+QZ_HD void cta_aed_deflate(X& x, WinState& w, double s, double* sr, double* si_, double* sb, int info, int nskip,
+                           bool swapfail, const HR& hessred) {
   int n = w.n;
-  x.stamp(0);
-  int info = ms ? cta_small_qz_ms(x, w, maxit, msscr) : cta_small_qz(x, w, maxit);
   x.stamp(1);
   if (info != 0) {
     // window QZ did not converge: deflate nothing, hand the diagonal
@@ -531,8 +531,22 @@ QZ_HD void cta_aed(X& x, WinState& w, double s, double* sr, double* si_, double*
     x.sync();
   }
   x.stamp(3);
-  cta_hessred(x, w, m);
+  if (!hessred(m)) {
+    if (x.tid == 0) { x.si[9] = n; x.si[10] = 0; }
+    x.sync();
+  }
   x.stamp(4);
+}
+
+template <class X>
+QZ_HD void cta_aed(X& x, WinState& w, double s, double* sr, double* si_, double* sb, int maxit, int nskip = 0,
+                   bool swapfail = false, double* msscr = nullptr) {
+  x.stamp(0);
+  const int info = msscr ? cta_small_qz_ms(x, w, maxit, msscr) : cta_small_qz(x, w, maxit);
+  cta_aed_deflate(x, w, s, sr, si_, sb, info, nskip, swapfail, [&](int m) {
+    cta_hessred(x, w, m);
+    return true;
+  });
 }
 
 }  // namespace qz

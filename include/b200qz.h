@@ -123,7 +123,7 @@ int b200qz_set_params(b200qz_ctx* ctx, int nw_max, int w_chase, int nmin, int ni
  * 0 = whole window), "max_wave" (chains chased concurrently, 1..8),
  * "stall_limit" (iterations without deflation before INFO > 0),
  * "split" (0, 7 or 8 INT8 Ozaki slices for the off-diagonal updates),
- * "aed_threads" (32, 64 or 128), "upd_persist" (0 or 1), "aed_limit"
+ * "aed_threads" (32, 64, 128 or 256), "upd_persist" (0 or 1), "aed_limit"
  * (stop before that AED, INFO 10003), "aed_swap_fail" (1: every block swap
  * inside the AED reports failure, which exercises the swap-failure branch
  * of the reference, qzearly.f:321-326).
