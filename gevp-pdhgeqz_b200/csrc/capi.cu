@@ -117,7 +117,8 @@ struct b200qz_ctx {
   int* ozerr = nullptr;        // device flag: a tensor-core wait timed out
   double* norms = nullptr;     // 2
   double* npart = nullptr;     // 592 per-block partial sums of the norm kernel
-  int* dinfo = nullptr;        // 16 ints: [4..6] AED info, [8..12] scan output
+  int* dinfo = nullptr;        // 16 ints: [4..6] AED info, [8..12] scan output, [13] a
+                               // wait inside a chase kernel gave up
   int* hinfo = nullptr;        // pinned mirror
   double* hshifts = nullptr;   // pinned 3*kAedMax
   double* hnorms = nullptr;    // pinned 2
@@ -187,8 +188,9 @@ struct GpuBackend {
     launch_scan(c->stream, H, T, ld, ifirst, kbot, tol, c->dinfo + 8);
     c->stats.launches += 1;
     c->timer.end(c->stream);
-    QZ_CK(cudaMemcpyAsync(c->hinfo, c->dinfo + 8, 5 * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    QZ_CK(cudaMemcpyAsync(c->hinfo, c->dinfo + 8, 6 * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     QZ_CK(cudaStreamSynchronize(c->stream));
+    if (c->err == cudaSuccess && c->hinfo[5] != 0) c->err = cudaErrorLaunchTimeout;
     if (c->err != cudaSuccess) { out[0] = ifirst; out[1] = 0; out[2] = -1; out[3] = -1; out[4] = 1; return; }
     for (int i = 0; i < 5; ++i) out[i] = c->hinfo[i];
   }
@@ -258,7 +260,7 @@ struct GpuBackend {
     }
     c->stats.chase_launches += 1;
     c->timer.begin(kPhChase, c->stream);
-    launch_chase_wave(c->stream, H, T, ld, wave, nw, c->Uc, c->Vc, kUslot);
+    launch_chase_wave(c->stream, H, T, ld, wave, nw, c->Uc, c->Vc, kUslot, c->dinfo + 13);
     c->timer.end(c->stream);
     c->stats.launches += 1;
     c->kc = kWinSmemMax;
@@ -479,6 +481,7 @@ int solve_dev_impl(b200qz_ctx* c, char job, char compq, char compz, int n, int i
   int nh = ihi - ilo + 1;
   // /PREC/ constants (PDHGEQZ.f:449-458): ulp, smlnum, Frobenius norms
   QZ_CK(cudaMemsetAsync(c->norms, 0, 2 * sizeof(double), c->stream));
+  QZ_CK(cudaMemsetAsync(c->dinfo + 13, 0, sizeof(int), c->stream));
   launch_sumsq(c->stream, h, ld, ilo - 1, nh, c->norms, c->npart);
   launch_sumsq(c->stream, t, ld, ilo - 1, nh, c->norms + 1, c->npart);
   c->stats.launches += 2;
@@ -804,9 +807,12 @@ int b200qz_chase_window(b200qz_ctx* c, double* h, double* t, int ld, int w, int 
     J.bl[b].c1 = coef[3 * b + 1];
     J.bl[b].c0 = coef[3 * b + 2];
   }
-  launch_chase_wave(c->stream, h, t, ld, wave, 1, u, v, 0);
+  QZ_CK(cudaMemsetAsync(c->dinfo + 13, 0, sizeof(int), c->stream));
+  launch_chase_wave(c->stream, h, t, ld, wave, 1, u, v, 0, c->dinfo + 13);
   QZ_CK(cudaGetLastError());
+  QZ_CK(cudaMemcpyAsync(c->hinfo, c->dinfo + 13, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   QZ_CK(cudaStreamSynchronize(c->stream));
+  if (c->err == cudaSuccess && c->hinfo[0] != 0) c->err = cudaErrorLaunchTimeout;
   return c->err == cudaSuccess ? 0 : 10001;
 }
 

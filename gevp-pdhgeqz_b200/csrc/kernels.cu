@@ -17,7 +17,7 @@
 #include <algorithm>
 
 #define QZ_DEFINE_UPDATE_KERNELS
-#include "qz_roles.cuh"
+#include "qz_chase_roles.cuh"
 #include "update.cuh"
 #include "kernels.h"
 
@@ -151,40 +151,41 @@ __global__ void __launch_bounds__(kThreads) k_aed_win(double* H, double* T, int6
 // ---------------------------------------------------------------------------
 // chase kernel
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kChaseThreads) k_chase_win(double* H, double* T, int64_t ld, const ChaseWave wave,
-                                                             double* Ug, double* Vg, int64_t ustride) {
+__global__ void __launch_bounds__(kChaseRoleThreads) k_chase_win(double* H, double* T, int64_t ld,
+                                                                 const ChaseWave wave, double* Ug, double* Vg,
+                                                                 int64_t ustride, int* err) {
   extern __shared__ double smem[];
   const ChaseJob& J = wave.job[blockIdx.x];
   const int w0 = J.w0, wk = J.wk, last = J.last, nb = J.nb, tmax = J.tmax;
   double* U = Ug + blockIdx.x * ustride;
   double* V = Vg + blockIdx.x * ustride;
-  const int lw = smem_ld(wk);
+  const int lw = smem_ld(wk), warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   double* Hs = smem;
   double* Ts = Hs + wk * lw;
   double* Us = Ts + wk * lw;
   double* Vs = Us + wk * lw;
-  Bulge* bl = (Bulge*)(Vs + wk * lw);
-  BulgeRec* rec = (BulgeRec*)(bl + kMaxChain);
-  int* si = (int*)(rec + kMaxChain);
-  DevExec x{(int)threadIdx.x, (int)blockDim.x, si, nullptr};
-  for (int idx = threadIdx.x; idx < wk * wk; idx += blockDim.x) {
-    int i = idx % wk, j = idx / wk;
-    Hs[i + j * lw] = G(H, ld, w0 + i, w0 + j);
-    Ts[i + j * lw] = G(T, ld, w0 + i, w0 + j);
-    Us[i + j * lw] = (i == j) ? 1.0 : 0.0;
-    Vs[i + j * lw] = (i == j) ? 1.0 : 0.0;
-  }
+  double* ring = Vs + wk * lw;  // 4 wk lw is even: 16-byte aligned
+  Bulge* bl = (Bulge*)(ring + chase_ring_doubles(nb));
+  ChaseShare* sh = (ChaseShare*)(bl + nb);
+  for (int j = warp; j < wk; j += nw)
+    for (int i = lane; i < wk; i += 32) {
+      Hs[i + j * lw] = G(H, ld, w0 + i, w0 + j);
+      Ts[i + j * lw] = G(T, ld, w0 + i, w0 + j);
+      Us[i + j * lw] = (i == j) ? 1.0 : 0.0;
+      Vs[i + j * lw] = (i == j) ? 1.0 : 0.0;
+    }
   for (int b = threadIdx.x; b < nb; b += blockDim.x) bl[b] = J.bl[b];
   __syncthreads();
-  cta_chase_window(x, wk, last, MatV{Hs, lw}, MatV{Ts, lw}, MatV{Us, lw}, MatV{Vs, lw}, bl, nb, tmax, rec);
-  __syncthreads();
-  for (int idx = threadIdx.x; idx < wk * wk; idx += blockDim.x) {
-    int i = idx % wk, j = idx / wk;
-    G(H, ld, w0 + i, w0 + j) = Hs[i + j * lw];
-    G(T, ld, w0 + i, w0 + j) = Ts[i + j * lw];
-    U[idx] = Us[i + j * lw];
-    V[idx] = Vs[i + j * lw];
-  }
+  const bool ok = cta_chase_roles(wk, last, MatV{Hs, lw}, MatV{Ts, lw}, MatV{Us, lw}, MatV{Vs, lw}, bl, nb, tmax, ring,
+                                  sh);
+  if (!ok && threadIdx.x == 0) *err = 1;
+  for (int j = warp; j < wk; j += nw)
+    for (int i = lane; i < wk; i += 32) {
+      G(H, ld, w0 + i, w0 + j) = Hs[i + j * lw];
+      G(T, ld, w0 + i, w0 + j) = Ts[i + j * lw];
+      U[i + j * wk] = Us[i + j * lw];
+      V[i + j * wk] = Vs[i + j * lw];
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -416,9 +417,13 @@ size_t aed_smem_bytes(int nw) {
   d += 64 + 4 * (size_t)nw + std::max(kMsScratch + kPipeDoubles, kRoleDoubles);
   return d * sizeof(double) + kSi * sizeof(int);
 }
+static size_t chase_smem_bytes(int wk, int nb);
 size_t chase_smem_bytes(int wk) {
-  return (size_t)4 * wk * smem_ld(wk) * sizeof(double) + kMaxChain * (sizeof(Bulge) + sizeof(BulgeRec)) +
-         kSi * sizeof(int);
+  return chase_smem_bytes(wk, kMaxChain);
+}
+static size_t chase_smem_bytes(int wk, int nb) {
+  return ((size_t)4 * wk * smem_ld(wk) + chase_ring_doubles(nb)) * sizeof(double) + nb * sizeof(Bulge) +
+         sizeof(ChaseShare);
 }
 size_t inf_smem_bytes(int wk) { return (size_t)4 * wk * smem_ld(wk) * sizeof(double) + kSi * sizeof(int); }
 
@@ -495,11 +500,11 @@ void launch_aed(cudaStream_t st, double* H, double* T, int64_t ld, int ktop, int
                                        nskip, swapfail, ms);
 }
 void launch_chase_wave(cudaStream_t st, double* H, double* T, int64_t ld, const ChaseWave& wave, int njob, double* U,
-                       double* V, int64_t ustride) {
+                       double* V, int64_t ustride, int* err) {
   if (njob <= 0) return;
-  int wmax = 0;
-  for (int i = 0; i < njob; ++i) wmax = wave.job[i].wk > wmax ? wave.job[i].wk : wmax;
-  k_chase_win<<<njob, kChaseThreads, chase_smem_bytes(wmax), st>>>(H, T, ld, wave, U, V, ustride);
+  size_t sm = 0;
+  for (int i = 0; i < njob; ++i) sm = std::max(sm, chase_smem_bytes(wave.job[i].wk, wave.job[i].nb));
+  k_chase_win<<<njob, kChaseRoleThreads, sm, st>>>(H, T, ld, wave, U, V, ustride, err);
 }
 void launch_inf(cudaStream_t st, double* H, double* T, int64_t ld, int w0, int wk, int top, int jz, int stop,
                 int deflate, double* U, double* V) {

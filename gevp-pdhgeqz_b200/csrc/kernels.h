@@ -9,7 +9,6 @@
 namespace qz {
 
 constexpr int kWinThreads = 128;   // threads of the one-CTA AED / zero-chase kernels
-constexpr int kChaseThreads = 512; // threads of the chase kernel
 constexpr int kWinSmemMax = 80;    // window size held entirely in shared memory (4 x 80^2 FP64 = 200 KB)
 constexpr int kMaxChain = 26;      // bulges per chain (3*26+2 rows fit a window of 80)
 
@@ -48,9 +47,10 @@ void launch_aed(cudaStream_t st, double* H, double* T, int64_t ld, int ktop, int
                 double* Qw, double* Zw, double* shifts, int* info, double* gscratch,
                 unsigned long long* ts = nullptr, int nskip = 0, int threads = kRoleThreads, int swapfail = 0,
                 int ms = 0);
-// one CTA per job; job i writes its factors to U + i*ustride, V + i*ustride
+// one CTA per job; job i writes its factors to U + i*ustride, V + i*ustride;
+// *err is set if a wait inside the kernel gave up
 void launch_chase_wave(cudaStream_t st, double* H, double* T, int64_t ld, const ChaseWave& wave, int njob, double* U,
-                       double* V, int64_t ustride);
+                       double* V, int64_t ustride, int* err);
 void launch_inf(cudaStream_t st, double* H, double* T, int64_t ld, int w0, int wk, int top, int jz, int stop,
                 int deflate, double* U, double* V);
 void launch_scan(cudaStream_t st, double* H, double* T, int64_t ld, int ifirst, int kbot, const Tol& tol, int* out);

@@ -23,12 +23,17 @@ namespace qz {
 // window limits allow; see piparmq.f:438-535).
 struct SolveParams {
   int nw_max = 48;       // AED window (one CTA, shared memory; up to 80)
-  int w_chase = 80;      // chase window
+  int w_chase = 64;      // chase window and bulges per chain: 64 and 8 (a bulge per
+                         // chase warp).  A step of the chase kernel costs 2,270
+                         // cycles there and 4,340 for 12 bulges in 80 rows, and the
+                         // shorter chains of a sweep run on more SMs at once:
+                         // chase + updates of an n=1800 solve 264 ms at (64, 8),
+                         // 381 at (80, 12), 281 at (48, 6), 329 at (32, 4)
   int nmin = 80;         // active blocks this small are solved by one CTA
   int nibble = -1;       // -1: table (14 in PDHGEQZ1 regime, 335*nh^-0.44 above)
   int ns_max = -1;       // -1: table
   int maxit_factor = 30; // MAXIT = 30*NH
-  int chain_max = -1;    // bulges per chain, -1: from w_chase
+  int chain_max = 8;     // -1: from w_chase
   int verbose = 0;       // progress lines on stderr (B200QZ_VERBOSE=1)
   int aed_nskip = -1;    // AED spike test stops after this many consecutive
                          // undeflatable blocks (0: test the whole window;
