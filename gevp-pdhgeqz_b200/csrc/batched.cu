@@ -9,10 +9,10 @@
 // decreasing size (longest-first scheduling), solve a pencil in shared
 // memory when n <= kBatchSmemMax (H, T, Q, Z with an odd leading
 // dimension), in place in global memory otherwise, normalise beta >= 0 and
-// write the eigenvalues.  Pencils long enough for chains of bulges are
-// reduced by small-bulge multishift sweeps (cta_small_qz_ms), shorter
-// ones by double-shift sweeps.  Per-pencil status words; no host round
-// trip.
+// write the eigenvalues.  Pencils in shared memory take the window QZ with
+// a role per warp (qz_roles.cuh: 3.8x the two-barrier sweeps at orders up to
+// 80); the others, and launches with 128 threads, small-bulge multishift
+// sweeps (cta_small_qz_ms).  Per-pencil status words; no host round trip.
 #include <cuda_runtime.h>
 #include <float.h>
 #include <stdint.h>
@@ -22,7 +22,7 @@
 
 #include "../../include/b200qz.h"
 #include "kernels.h"
-#include "qz_window.cuh"
+#include "qz_roles.cuh"
 
 namespace qz {
 
@@ -119,7 +119,10 @@ __global__ void __launch_bounds__(kBatchThreads) k_batch_qz(int count, const int
       }
     }
     __syncthreads();
-    BExec x{(int)threadIdx.x, (int)blockDim.x, si, sd_small};
+    // role-per-warp QZ: its buffer and scratch behind the matrices
+    const bool roles = in_smem && blockDim.x == kRoleThreads;
+    RoleBuf* const rb = (RoleBuf*)(smem + 4 * smem_max * smem_ld(smem_max));
+    BExec x{(int)threadIdx.x, (int)blockDim.x, si, roles ? (double*)(rb + 1) : sd_small};
     WinState w;
     w.n = n;
     w.H = MatV{Hs, lw};
@@ -129,8 +132,17 @@ __global__ void __launch_bounds__(kBatchThreads) k_batch_qz(int count, const int
     w.wantq = true;
     w.wantz = true;
     w.tol = tol;
-    // pencils long enough for chains of bulges take multishift sweeps
-    int info = cta_small_qz_ms(x, w, 30 * n, ms_scr);
+    int info;
+    if (roles) {
+      w.H.p = smem;  // (shared-memory accesses throughout)
+      w.T.p = smem + n * lw;
+      w.Q.p = smem + 2 * n * lw;
+      w.Z.p = smem + 3 * n * lw;
+      info = cta_role_qz(x, w, 30 * n, rb);
+      if (info == 0) cta_std_all(x, w, x.sd);
+    } else {
+      info = cta_small_qz_ms(x, w, 30 * n, ms_scr);
+    }
     __syncthreads();
     if (info == 0) cta_finalize(x, w, AR + eoff[p], AI + eoff[p], BE + eoff[p]);
     if (in_smem) {
@@ -147,7 +159,10 @@ __global__ void __launch_bounds__(kBatchThreads) k_batch_qz(int count, const int
   }
 }
 
-size_t batch_smem_bytes(int smem_max) { return (size_t)4 * smem_max * smem_ld(smem_max) * sizeof(double); }
+// H, T, Q, Z, then the role buffer and the standardisation's 3n doubles
+size_t batch_smem_bytes(int smem_max) {
+  return ((size_t)4 * smem_max * smem_ld(smem_max) + kRoleDoubles + 3 * (size_t)smem_max) * sizeof(double);
+}
 
 cudaError_t batch_init() {
   return cudaFuncSetAttribute(k_batch_qz, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -262,7 +277,7 @@ extern "C" int b200qz_solve_batched_noalloc(int count, const int* n, const long 
       cudaMemcpyAsync(d_n, n, count * sizeof(int), cudaMemcpyHostToDevice, st) != cudaSuccess)
     return 10001;
   // the queue counter is zeroed on the stream before the kernel starts
-  const cudaError_t e = launch_batch_checked(st, d->sm_count, 128, kBatchSmemMax, count, d_order, d_n, d_moff, d_eoff,
+  const cudaError_t e = launch_batch_checked(st, d->sm_count, kRoleThreads, kBatchSmemMax, count, d_order, d_n, d_moff, d_eoff,
                                              h, t, q, z, alphar, alphai, beta, info, d_counter);
   return e == cudaSuccess ? 0 : 10001;
 }

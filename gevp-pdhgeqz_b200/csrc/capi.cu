@@ -137,7 +137,7 @@ struct b200qz_ctx {
   // batched solver
   int* bdesc = nullptr;                // device: order, n, counter, moff/eoff (int64) packed
   size_t bdesc_bytes = 0;
-  int batch_threads = 128, batch_smem_max = kBatchSmemMax, batch_ctas_per_sm = 1;
+  int batch_threads = kRoleThreads, batch_smem_max = kBatchSmemMax, batch_ctas_per_sm = 1;
   cudaGraph_t bgraph = nullptr;
   cudaGraphExec_t bexec = nullptr;
   BatchKey bkey;                       // operands and configuration of the captured launch
