@@ -4,18 +4,23 @@
 // windowed reordering PDTGORD (src/reorder/PDTGSEN.f:1, PDTGORD.f:1;
 // used after the solve at examples/EXRAND3.f:473).
 //
-// Moves.  The selected blocks are taken in order from the top; each moves
-// up to the next free position through windows of at most 80 rows.  One
-// CTA holds a window's S and T in shared memory, swaps the block up to the
-// window's top by adjacent block swaps (the generalized Sylvester swap of
-// the AED, cta_swap, standardising the 2x2 blocks it moves) and
-// accumulates the window's orthogonal factors U, V; the DMMA update
-// kernels then apply U, V to the rest of S, T and to Q, Z.  The host keeps
-// the block structure (sizes in order), so windows start at block
-// boundaries without reading the matrices back.  A rejected swap sets a
-// device flag: later windows leave their pencil unchanged (identity
-// factors) and the call returns info = 1 with the partly reordered form,
-// as DTGSEN does.
+// Moves.  reorder_plan.h lays out a stable partition of the diagonal blocks
+// by adjacent swaps: phases of disjoint windows of at most 80 rows, a CTA per
+// window, and inside a window rounds of disjoint swaps.  A CTA holds its
+// window's S and T in shared memory; a round forms all its swaps at once (a
+// thread per swap, by the generalized Sylvester equation of the AED's
+// swaps), applies their left factors, then their right ones, and accumulates
+// them in the window's U and V; the 2x2 blocks are standardised once at the
+// end of the window.  The DMMA update kernels then apply U, V to the rest of
+// S, T and to Q, Z, all windows of a phase in one left and one right batch.
+// The host knows every position in advance, so no launch waits for another's
+// outcome.  A rejected swap sets a device flag: its window ends with the
+// round, later windows leave their pencil unchanged (identity factors) and
+// the call returns info = 1 with the partly reordered form, as DTGSEN does.
+//
+// Bound: a swap's serial computation (about 5,000 cycles for two 2x2
+// blocks), once per round; one block moved at a time, as DTGSEN does, has
+// the same number of swaps in sequence.
 //
 // Normalisation.  A 1x1 block whose T entry is negative has its rows of S
 // and T and its column of Q negated (DTGSEN's convention); the eigenvalues
@@ -36,18 +41,19 @@
 // Gaussian elimination with complete pivoting.
 #include "reorder.h"
 
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 #include <vector>
 
 #include "kernels.h"
 #include "onenorm.h"
+#include "reorder_plan.h"
 
 namespace qz {
 namespace {
 
-constexpr int kReoWin = 80;  // window rows (shared memory)
-constexpr int kReoThreads = 128;
+constexpr int kReoThreads = 256;
 
 struct ReoExec {
   int tid, nt;
@@ -58,70 +64,165 @@ struct ReoExec {
   __device__ void count(int) {}
 };
 
-size_t reo_smem(int wk) { return ((size_t)4 * wk * smem_ld(wk) + 256) * sizeof(double) + 64 * sizeof(int); }
+// S, T, U, V of the window, Q, Z, S2, T2 (16 each) of a round's swaps (the
+// standardisation's 3n doubles reuse them), their status
+constexpr int kReoRec = 64;
+size_t reo_smem(int wk) {
+  return ((size_t)4 * wk * smem_ld(wk) + (size_t)(wk / 2 + 1) * kReoRec + 3 * wk) * sizeof(double) +
+         (kReoPairs + 8) * sizeof(int);
+}
 
-// Move the block at window row ifst (size bs) up to window row 0 of the
-// window S(w0:w0+wk, w0:w0+wk); U, V receive the window's factors.
-// status = {failed, global row where the block stopped}.
-__global__ void __launch_bounds__(kReoThreads) k_reorder_win(double* S, int64_t lds, double* T, int64_t ldt, int w0,
-                                                             int wk, int ifst, int bs, Tol tol, double* U, double* V,
+// one swap of blocks of sizes N1, N2 at window row j, by one thread, to rec
+template <int N1, int N2>
+__device__ __forceinline__ bool reo_swap(double* S, double* T, int ld, int j, const Tol& tol, double* rec) {
+  constexpr int M = N1 + N2;
+  const MatV hb{S + j + j * ld, ld}, tb{T + j + j * ld, ld};
+  double S2[M * M], T2[M * M], Qs[M * M], Zs[M * M];
+  int res;
+  if constexpr (N1 == 1 && N2 == 1)
+    // two rotations; the Sylvester path where they fail the stability test
+    res = swap_compute11(hb, tb, S2, T2, Qs, Zs, tol.ulp, tol.smlnum)
+              ? 1
+              : swap_compute_try<1, 1>(hb, tb, S2, T2, Qs, Zs, tol.ulp, tol.smlnum);
+  else
+    res = swap_compute_try<N1, N2>(hb, tb, S2, T2, Qs, Zs, tol.ulp, tol.smlnum);
+  if (res > 0) {
+#pragma unroll
+    for (int i = 0; i < M * M; ++i) { rec[i] = Qs[i]; rec[16 + i] = Zs[i]; rec[32 + i] = S2[i]; rec[48 + i] = T2[i]; }
+    return true;
+  }
+  return res < 0 && swap_retry<N1, N2>(hb, tb, rec + 32, rec + 48, rec, rec + 16, tol.ulp, tol.smlnum);
+}
+
+// y = F^T x (rows) or x F (columns) for the M entries at p, p + st, ..: the
+// same sums, F = Q or Z
+template <int M>
+__device__ __forceinline__ void reo_line(const double* f, double* p, int st) {
+  double x[M];
+#pragma unroll
+  for (int i = 0; i < M; ++i) x[i] = p[i * st];
+#pragma unroll
+  for (int c = 0; c < M; ++c) {
+    double a = 0.0;
+#pragma unroll
+    for (int k = 0; k < M; ++k) a += x[k] * f[k + M * c];
+    p[c * st] = a;
+  }
+}
+__device__ __forceinline__ void reo_line_any(int m, const double* f, double* p, int st) {
+  if (m == 2) reo_line<2>(f, p, st);
+  else if (m == 3) reo_line<3>(f, p, st);
+  else reo_line<4>(f, p, st);
+}
+
+// One window per CTA; status[1] is set when a swap is rejected.  A 2x2 block
+// whose eigenvalues turn out real keeps moving as one.
+__global__ void __launch_bounds__(kReoThreads) k_reorder_win(double* S, int64_t lds, double* T, int64_t ldt,
+                                                             const ReoWindow* wins, const int* rounds,
+                                                             const int* swaps, Tol tol, double* Ug, double* Vg,
                                                              int* status) {
   extern __shared__ double smem[];
-  const int lw = smem_ld(wk);
+  const ReoWindow W = wins[blockIdx.x];
+  const int wk = W.wk, w0 = W.w0, ld = smem_ld(wk);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
   double* Hs = smem;
-  double* Ts = Hs + wk * lw;
-  double* Us = Ts + wk * lw;
-  double* Vs = Us + wk * lw;
-  double* sd = Vs + wk * lw;
-  int* si = (int*)(sd + 256);
-  const bool skip = *(volatile int*)status != 0;  // an earlier window was rejected
-  for (int idx = threadIdx.x; idx < wk * wk; idx += blockDim.x) {
-    const int i = idx % wk, j = idx / wk;
-    if (!skip) {
-      Hs[i + j * lw] = S[(w0 + i) + (int64_t)(w0 + j) * lds];
-      Ts[i + j * lw] = T[(w0 + i) + (int64_t)(w0 + j) * ldt];
+  double* Ts = Hs + wk * ld;
+  double* Us = Ts + wk * ld;
+  double* Vs = Us + wk * ld;
+  double* recs = Vs + wk * ld;
+  int* good = (int*)(recs + (wk / 2 + 1) * kReoRec + 3 * wk);
+  int* bad = good + kReoPairs;
+  double* const U = Ug + (size_t)blockIdx.x * kReoWin * kReoWin;
+  double* const V = Vg + (size_t)blockIdx.x * kReoWin * kReoWin;
+  // an earlier phase's window was rejected (this phase's set the second word)
+  const bool skip = *(volatile int*)status != 0;
+  if (tid == 0) *bad = 0;
+  for (int j = warp; j < wk; j += nw)
+    for (int i = lane; i < wk; i += 32) {
+      if (!skip) {
+        Hs[i + j * ld] = S[(w0 + i) + (int64_t)(w0 + j) * lds];
+        Ts[i + j * ld] = T[(w0 + i) + (int64_t)(w0 + j) * ldt];
+      }
+      Us[i + j * ld] = (i == j) ? 1.0 : 0.0;
+      Vs[i + j * ld] = (i == j) ? 1.0 : 0.0;
     }
-    Us[i + j * lw] = (i == j) ? 1.0 : 0.0;
-    Vs[i + j * lw] = (i == j) ? 1.0 : 0.0;
-  }
   __syncthreads();
   if (!skip) {
-    ReoExec x{(int)threadIdx.x, (int)blockDim.x, si, sd};
+    for (int r = 0; r < W.rounds; ++r) {
+      const int s0 = rounds[W.r0 + r], np = rounds[W.r0 + r + 1] - s0;
+      // a thread per swap, the four kinds on four warps
+      if (warp < 4)
+        for (int k = lane; k < np; k += 32) {
+          const int sw = swaps[s0 + k], j = sw & 255, n1 = (sw >> 8) & 15, n2 = sw >> 12;
+          if (2 * (n1 - 1) + n2 - 1 != warp) continue;
+          double* const rec = recs + k * kReoRec;
+          bool ok;
+          if (warp == 0) ok = reo_swap<1, 1>(Hs, Ts, ld, j, tol, rec);
+          else if (warp == 1) ok = reo_swap<1, 2>(Hs, Ts, ld, j, tol, rec);
+          else if (warp == 2) ok = reo_swap<2, 1>(Hs, Ts, ld, j, tol, rec);
+          else ok = reo_swap<2, 2>(Hs, Ts, ld, j, tol, rec);
+          good[k] = ok;
+          if (!ok) *bad = 1;
+        }
+      __syncthreads();
+      // left factors: rows of S, T right of the block; columns of U
+      for (int k = warp; k < np; k += nw) {
+        if (!good[k]) continue;
+        const int sw = swaps[s0 + k], j = sw & 255, m = ((sw >> 8) & 15) + (sw >> 12);
+        const double* const rec = recs + k * kReoRec;
+        for (int c = j + m + lane; c < wk; c += 32) {
+          reo_line_any(m, rec, Hs + j + c * ld, 1);
+          reo_line_any(m, rec, Ts + j + c * ld, 1);
+        }
+        for (int i = lane; i < wk; i += 32) reo_line_any(m, rec, Us + i + j * ld, ld);
+      }
+      __syncthreads();
+      // right factors: columns of S, T above the block; columns of V; the block
+      for (int k = warp; k < np; k += nw) {
+        if (!good[k]) continue;
+        const int sw = swaps[s0 + k], j = sw & 255, m = ((sw >> 8) & 15) + (sw >> 12);
+        const double* const rec = recs + k * kReoRec;
+        for (int i = lane; i < j; i += 32) {
+          reo_line_any(m, rec + 16, Hs + i + j * ld, ld);
+          reo_line_any(m, rec + 16, Ts + i + j * ld, ld);
+        }
+        for (int i = lane; i < wk; i += 32) reo_line_any(m, rec + 16, Vs + i + j * ld, ld);
+        if (lane < m * m) {
+          Hs[j + lane % m + (j + lane / m) * ld] = rec[32 + lane];
+          Ts[j + lane % m + (j + lane / m) * ld] = rec[48 + lane];
+        }
+      }
+      __syncthreads();
+      if (*bad) break;
+    }
+    ReoExec x{tid, (int)blockDim.x, nullptr, recs};
     WinState w;
     w.n = wk;
-    w.H = MatV{Hs, lw};
-    w.T = MatV{Ts, lw};
-    w.Q = MatV{Us, lw};
-    w.Z = MatV{Vs, lw};
+    w.H = MatV{Hs, ld};
+    w.T = MatV{Ts, ld};
+    w.Q = MatV{Us, ld};
+    w.Z = MatV{Vs, ld};
     w.wantq = true;
     w.wantz = true;
     w.tol = tol;
-    int here = ifst;
-    bool ok = true;
-    while (here > 0) {
-      int nbn = 1;
-      if (here >= 2 && w.H(here - 1, here - 2) != 0.0) nbn = 2;
-      if (!cta_swap(x, w, here - nbn, nbn, bs, true)) { ok = false; break; }
-      here -= nbn;
-      const int nbnow = (bs == 2 && w.H(here + 1, here) != 0.0) ? 2 : 1;
-      if (nbnow != bs) { ok = false; break; }
-    }
-    __syncthreads();
-    if (!ok && threadIdx.x == 0) {
-      status[0] = 1;
-      status[1] = w0 + here;
-    }
-    for (int idx = threadIdx.x; idx < wk * wk; idx += blockDim.x) {
-      const int i = idx % wk, j = idx / wk;
-      S[(w0 + i) + (int64_t)(w0 + j) * lds] = Hs[i + j * lw];
-      T[(w0 + i) + (int64_t)(w0 + j) * ldt] = Ts[i + j * lw];
-    }
+    cta_std_all(x, w, recs);
+    if (tid == 0 && *bad) status[1] = 1;
+    for (int j = warp; j < wk; j += nw)
+      for (int i = lane; i < wk; i += 32) {
+        S[(w0 + i) + (int64_t)(w0 + j) * lds] = Hs[i + j * ld];
+        T[(w0 + i) + (int64_t)(w0 + j) * ldt] = Ts[i + j * ld];
+      }
   }
-  for (int idx = threadIdx.x; idx < wk * wk; idx += blockDim.x) {
-    const int i = idx % wk, j = idx / wk;
-    U[idx] = Us[i + j * lw];
-    V[idx] = Vs[i + j * lw];
-  }
+  for (int j = warp; j < wk; j += nw)
+    for (int i = lane; i < wk; i += 32) {
+      U[i + j * wk] = Us[i + j * ld];
+      V[i + j * wk] = Vs[i + j * ld];
+    }
+}
+
+// after a phase: its rejections hold for the next ones
+__global__ void k_reorder_status(int* status) {
+  if (status[1]) status[0] = 1;
 }
 
 // 1x1 blocks with a negative T entry: rows of S and T and column of Q negated
@@ -548,66 +649,68 @@ cudaError_t tgsen_device(cudaStream_t st, int ijob, bool wantq, bool wantz, cons
   tol.ttol = DBL_MIN;
   tol.htol = DBL_MIN;
 
+  ReoPlan plan;
+  reorder_plan(sz, sel, plan);
   DevMem mem;
-  e = cudaMalloc(&mem.p, sizeof(double) * 2 * kReoWin * kReoWin + 64);
-  if (e != cudaSuccess) return e;
-  double* U = (double*)mem.p;
-  double* V = U + kReoWin * kReoWin;
-  int* status = (int*)(V + kReoWin * kReoWin);
-  e = cudaMemsetAsync(status, 0, 2 * sizeof(int), st);
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_reorder_win, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)reo_smem(kReoWin));
-  if (e != cudaSuccess) return e;
-
-  int ks = 0, bks = 0;  // next free row and block index
-  for (int b = 0; b < nb && out->info == 0; ++b) {
-    if (!sel[b]) continue;
-    int pos = ks;
-    for (int k = bks; k < b; ++k) pos += sz[k];
-    const int bs = sz[b];
-    int ci = b;
-    while (ci > bks) {
-      // window: from the first block boundary within kReoWin rows of the
-      // block's end down to the block's end
-      int ti = ci, tpos = pos;
-      while (ti > bks && (pos + bs) - (tpos - sz[ti - 1]) <= kReoWin) tpos -= sz[--ti];
-      const int wk = pos + bs - tpos;
-      k_reorder_win<<<1, kReoThreads, reo_smem(wk), st>>>(S, lds, T, ldt, tpos, wk, pos - tpos, bs, tol, U, V,
-                                                          status);
-      UpdBatch L, R;
-      L.njobs = 0;
-      R.njobs = 0;
-      add_job(L, S, lds, tpos, tpos + wk, n - (tpos + wk), U, wk);
-      add_job(L, T, ldt, tpos, tpos + wk, n - (tpos + wk), U, wk);
-      add_job(R, S, lds, 0, tpos, tpos, V, wk);
-      add_job(R, T, ldt, 0, tpos, tpos, V, wk);
-      if (wantq) add_job(R, Q, ldq, 0, tpos, n, U, wk);
-      if (wantz) add_job(R, Z, ldz, 0, tpos, n, V, wk);
-      if (L.njobs) launch_update(st, L, 0);
-      if (R.njobs) launch_update(st, R, 1);
+  if (!plan.phase.empty()) {
+    const size_t fac = (size_t)plan.most * kReoWin * kReoWin;
+    const size_t nwin = plan.win.size() * sizeof(ReoWindow), nround = plan.round.size() * sizeof(int),
+                 nswap = plan.swap.size() * sizeof(int);
+    e = cudaMalloc(&mem.p, 2 * fac * sizeof(double) + nwin + nround + nswap + 2 * sizeof(int));
+    if (e != cudaSuccess) return e;
+    double* U = (double*)mem.p;
+    double* V = U + fac;
+    ReoWindow* dwin = (ReoWindow*)(V + fac);
+    int* dround = (int*)(dwin + plan.win.size());
+    int* dswap = dround + plan.round.size();
+    int* status = dswap + plan.swap.size();
+    e = cudaMemsetAsync(status, 0, 2 * sizeof(int), st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(dwin, plan.win.data(), nwin, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(dround, plan.round.data(), nround, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(dswap, plan.swap.data(), nswap, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k_reorder_win, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)reo_smem(kReoWin));
+    if (e != cudaSuccess) return e;
+    for (const ReoPhase& F : plan.phase) {
+      int wmax = 0;
+      for (int i = 0; i < F.count; ++i) wmax = std::max(wmax, plan.win[F.first + i].wk);
+      k_reorder_win<<<F.count, kReoThreads, reo_smem(wmax), st>>>(S, lds, T, ldt, dwin + F.first, dround, dswap, tol,
+                                                                  U, V, status);
+      k_reorder_status<<<1, 1, 0, st>>>(status);
+      // every left update of the phase before every right one
+      for (int side = 0; side < 2; ++side) {
+        UpdBatch B;
+        B.njobs = 0;
+        for (int i = 0; i < F.count; ++i) {
+          const ReoWindow& w = plan.win[F.first + i];
+          const double* u = U + (size_t)i * kReoWin * kReoWin;
+          const double* v = V + (size_t)i * kReoWin * kReoWin;
+          if (B.njobs + 4 > kUpdMaxJobs) {
+            launch_update(st, B, side);
+            B.njobs = 0;
+          }
+          if (side == 0) {
+            add_job(B, S, lds, w.w0, w.w0 + w.wk, n - (w.w0 + w.wk), u, w.wk);
+            add_job(B, T, ldt, w.w0, w.w0 + w.wk, n - (w.w0 + w.wk), u, w.wk);
+          } else {
+            add_job(B, S, lds, 0, w.w0, w.w0, v, w.wk);
+            add_job(B, T, ldt, 0, w.w0, w.w0, v, w.wk);
+            if (wantq) add_job(B, Q, ldq, 0, w.w0, n, u, w.wk);
+            if (wantz) add_job(B, Z, ldz, 0, w.w0, n, v, w.wk);
+          }
+        }
+        if (B.njobs) launch_update(st, B, side);
+      }
       e = cudaGetLastError();
       if (e != cudaSuccess) return e;
-      out->windows += 1;
-      out->swaps += ci - ti;
-      // the block now leads the window
-      for (int k = ci; k > ti; --k) {
-        std::swap(sz[k], sz[k - 1]);
-        std::swap(sel[k], sel[k - 1]);
-      }
-      ci = ti;
-      pos = tpos;
     }
+    out->windows = (int)plan.win.size();
+    out->swaps = (int)plan.swaps;
     int hs[2] = {0, 0};
     e = cudaMemcpyAsync(hs, status, sizeof(hs), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return e;
-    e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return e;
-    if (hs[0]) {
-      out->info = 1;
-      break;
-    }
-    ks += bs;
-    ++bks;
+    if (hs[1]) out->info = 1;
   }
   k_tgsen_signs<<<n, 256, 0, st>>>(S, lds, T, ldt, Q, ldq, n, wantq ? 1 : 0);
   k_tgsen_eigs<<<(n + 255) / 256, 256, 0, st>>>(S, lds, T, ldt, n, alphar, alphai, beta);
