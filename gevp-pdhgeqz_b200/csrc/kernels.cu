@@ -436,8 +436,8 @@ static size_t upd_smem(int k, int side) {
 
 static size_t upd_smem_persist(int k, int side) {
   int kp = (k + 15) & ~15;
-  if (side == 0) return ((size_t)kp * (kp + 4) + 2 * (size_t)kp * 36) * sizeof(double);
-  return ((size_t)kp * (kp + 4) + 2 * (size_t)kUpdTile * (kp + 4)) * sizeof(double);
+  if (side == 0) return ((size_t)kp * (kp + 4) + 2 * (size_t)kUpdTile * (kp + 4)) * sizeof(double);
+  return ((size_t)kp * (kp + 4) + 2 * (size_t)kp * kUpdRightLd) * sizeof(double);
 }
 
 static int g_sm_count = 0;
@@ -534,8 +534,8 @@ void launch_update(cudaStream_t st, const UpdBatch& B_in, int side, int persist)
     per_sm = per_sm < 1 ? 1 : (per_sm > 4 ? 4 : per_sm);
     int grid = (g_sm_count > 0 ? g_sm_count : 148) * per_sm;
     if (grid > tiles) grid = tiles;
-    // one warp per 16-row (left) / 16-column (right) slice of the largest window
-    int warps = ((B.k + 15) & ~15) / 16;
+    // two warps per 16-row (left) / 16-column (right) slice of the largest window
+    int warps = ((B.k + 15) & ~15) / 8;
     warps = warps < 1 ? 1 : (warps > kUpdMaxThreads / 32 ? kUpdMaxThreads / 32 : warps);
     if (side == 0) k_update_persist<0><<<grid, 32 * warps, sm, st>>>(B, tiles);
     else k_update_persist<1><<<grid, 32 * warps, sm, st>>>(B, tiles);

@@ -39,7 +39,7 @@ struct UpdBatch {
 
 constexpr int kUpdTile = 32;       // slab tile width (columns for left, rows for right)
 constexpr int kUpdThreads = 128;   // 4 warps (per-tile kernels)
-constexpr int kUpdMaxThreads = 256;  // persistent kernels: one warp per 16-row slice, up to 8
+constexpr int kUpdMaxThreads = 512;  // persistent kernels: two warps per 16-row slice, up to 16
 constexpr int kUpdMaxK = 128;      // fast path limit
 
 #ifdef QZ_DEFINE_UPDATE_KERNELS
@@ -196,11 +196,22 @@ __global__ void __launch_bounds__(kUpdThreads) k_update_right(UpdBatch B) {
 // run of tiles, keeps the k x k factor in shared memory while consecutive
 // tiles belong to the same job, and prefetches the next slab tile with
 // cp.async into a second buffer while the current one is multiplied.
+//
+// Factor and tile are copied as they lie in memory (runs of a column), in
+// 16-byte pieces where the run starts on 16 bytes, and the fragments are
+// read from that layout without bank conflicts (leading dimensions 4 mod 16
+// doubles):
+//   factor  Wm[j][i] = W(i, j);  left tile Xs[j][i];  right tile Xs[kk][i].
+// A launch of the solver has a tile or two per CTA, so what bounds it is this
+// prologue: with element-wise transposing copies a wave's updates at
+// n=1800 (k=64) took 21 us a launch.
+// Two warps share a 16-row (16-column) slice of the product, half of its
+// columns (rows) each.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void upd_cp8(void* sdst, const void* gsrc, bool valid) {
+__device__ __forceinline__ void upd_cp(void* sdst, const void* gsrc, int bytes) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(sdst);
-  const int sz = valid ? 8 : 0;  // 0: zero-fill, nothing read
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(gsrc), "r"(sz) : "memory");
+  if (bytes == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gsrc) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gsrc) : "memory");
 }
 __device__ __forceinline__ void upd_cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
@@ -215,37 +226,56 @@ __device__ __forceinline__ int upd_locate(const UpdBatch& B, int t, int& tile) {
   return -1;
 }
 
-// stage slab tile `tile` of job J into Xs (layout as in the kernels above)
-__device__ __forceinline__ void upd_stage(const UpdJob& J, int tile, int side, double* Xs, int kpmax) {
-  const int k = J.k;
-  const int kp = (k + 15) & ~15;
-  if (side == 0) {
-    const int c0 = J.c0 + tile * kUpdTile;
-    const int ncol = min(kUpdTile, J.c0 + J.len - c0);
-    for (int idx = threadIdx.x; idx < kp * kUpdTile; idx += blockDim.x) {
-      const int kk = idx % kp, j = idx / kp;
-      const bool v = kk < k && j < ncol;
-      upd_cp8(&Xs[kk * 36 + j], v ? &J.M[(J.r0 + kk) + (int64_t)(c0 + j) * J.ld] : J.M, v);
-    }
-  } else {
-    const int r0 = J.r0 + tile * kUpdTile;
-    const int nrow = min(kUpdTile, J.r0 + J.len - r0);
-    const int ldx = kpmax + 4;
-    for (int idx = threadIdx.x; idx < kUpdTile * kp; idx += blockDim.x) {
-      const int i = idx % kUpdTile, kk = idx / kUpdTile;
-      const bool v = i < nrow && kk < k;
-      upd_cp8(&Xs[i * ldx + kk], v ? &J.M[(r0 + i) + (int64_t)(J.c0 + kk) * J.ld] : J.M, v);
+// runs of `len` doubles at src + r ld (r < runs) to dst + r dld, the rest of
+// `plen` x `pruns` zero; half a warp per run
+__device__ __forceinline__ void upd_copy(double* dst, int dld, const double* src, int64_t ld, int len, int runs,
+                                         int plen, int pruns) {
+  const int l = threadIdx.x & 15, g = threadIdx.x >> 4, ng = blockDim.x >> 4;
+  const bool wide = (((uintptr_t)src | (uintptr_t)(ld * 8)) & 15) == 0;
+  for (int r = g; r < pruns; r += ng) {
+    double* const d = dst + r * dld;
+    const double* const q = src + r * ld;
+    const int n = r < runs ? len : 0;
+    if (wide) {
+      for (int i = 2 * l; i < plen; i += 32) {
+        if (i + 1 < n) {
+          upd_cp(d + i, q + i, 16);
+        } else {
+          d[i] = i < n ? q[i] : 0.0;
+          d[i + 1] = 0.0;
+        }
+      }
+    } else {
+      for (int i = l; i < plen; i += 16) {
+        if (i < n) upd_cp(d + i, q + i, 8);
+        else d[i] = 0.0;
+      }
     }
   }
 }
+
+// stage slab tile `tile` of job J into Xs
+__device__ __forceinline__ void upd_stage(const UpdJob& J, int tile, int side, double* Xs, int ldx) {
+  const int kp = (J.k + 15) & ~15;
+  if (side == 0) {
+    const int c0 = J.c0 + tile * kUpdTile;
+    upd_copy(Xs, ldx, J.M + J.r0 + (int64_t)c0 * J.ld, J.ld, J.k, min(kUpdTile, J.c0 + J.len - c0), kp, kUpdTile);
+  } else {
+    const int r0 = J.r0 + tile * kUpdTile;
+    upd_copy(Xs, ldx, J.M + r0 + (int64_t)J.c0 * J.ld, J.ld, min(kUpdTile, J.r0 + J.len - r0), J.k, kUpdTile, kp);
+  }
+}
+
+constexpr int kUpdRightLd = kUpdTile + 4;
 
 template <int SIDE>
 __global__ void __launch_bounds__(kUpdMaxThreads) k_update_persist(UpdBatch B, int total) {
   extern __shared__ double smem[];
   const int kpmax = (B.k + 15) & ~15;
   const int ldw = kpmax + 4;
+  const int ldx = SIDE == 0 ? ldw : kUpdRightLd;
   double* Wm = smem;                                  // kpmax x (kpmax + 4)
-  const int xsz = SIDE == 0 ? kpmax * 36 : kUpdTile * (kpmax + 4);
+  const int xsz = SIDE == 0 ? kUpdTile * ldx : kpmax * ldx;
   double* const Xbase = smem + kpmax * ldw;         // two slab buffers of xsz
   const int chunk = (total + gridDim.x - 1) / gridDim.x;
   const int t0 = blockIdx.x * chunk;
@@ -254,24 +284,20 @@ __global__ void __launch_bounds__(kUpdMaxThreads) k_update_persist(UpdBatch B, i
   const int tid = threadIdx.x;
   int tile_next;
   int jb_next = upd_locate(B, t0, tile_next);
-  upd_stage(B.job[jb_next], tile_next, SIDE, Xbase, kpmax);
-  upd_cp_commit();
   int cur = -1;
+  bool staged = false;  // tile t is on its way already
   for (int t = t0; t < t1; ++t) {
     const int jb = jb_next, tile = tile_next;
     const UpdJob J = B.job[jb];
     const int k = J.k;
     const int kp = (k + 15) & ~15;
     if (jb != cur) {
-      // factor of this job (W^T for the left update)
-      for (int idx = tid; idx < kp * kp; idx += blockDim.x) {
-        const int a = idx % kp, b = idx / kp;
-        const double v = (a < k && b < k) ? J.W[a + (int64_t)b * J.ldw] : 0.0;
-        if (SIDE == 0) Wm[b * ldw + a] = v;   // Wt[i][kk] = W(kk, i)
-        else Wm[a * ldw + b] = v;             // Ws[kk][j] = W(kk, j)
-      }
+      // factor of this job
+      upd_copy(Wm, ldw, J.W, J.ldw, k, k, kp, kp);
       cur = jb;
     }
+    if (!staged) upd_stage(J, tile, SIDE, Xbase + ((t - t0) & 1) * xsz, ldx);
+    upd_cp_commit();
     if (t + 1 < t1) {
       // next tile (the next job's tile if this one is done)
       if (tile + 1 < B.job[jb].tiles) { jb_next = jb; tile_next = tile + 1; }
@@ -280,7 +306,8 @@ __global__ void __launch_bounds__(kUpdMaxThreads) k_update_persist(UpdBatch B, i
         tile_next = 0;
         while (jb_next < B.njobs - 1 && B.job[jb_next].tiles == 0) ++jb_next;
       }
-      upd_stage(B.job[jb_next], tile_next, SIDE, Xbase + ((t + 1 - t0) & 1) * xsz, kpmax);
+      upd_stage(B.job[jb_next], tile_next, SIDE, Xbase + ((t + 1 - t0) & 1) * xsz, ldx);
+      staged = true;
       upd_cp_commit();
       upd_cp_wait<1>();
     } else {
@@ -290,72 +317,46 @@ __global__ void __launch_bounds__(kUpdMaxThreads) k_update_persist(UpdBatch B, i
     const double* Xs = Xbase + ((t - t0) & 1) * xsz;
     const int warp = tid >> 5, lane = tid & 31;
     const int lr = lane >> 2, lc = lane & 3;
-    const int nslice = kp / 16;
-    if (SIDE == 0) {
-      const int c0 = J.c0 + tile * kUpdTile;
-      const int ncol = min(kUpdTile, J.c0 + J.len - c0);
-      for (int sl = warp; sl < nslice; sl += (int)(blockDim.x >> 5)) {
-        double acc[2][4][2];
+    const int half = warp & 1, nslice = kp / 16;
+    for (int sl = warp >> 1; sl < nslice; sl += (int)(blockDim.x >> 6)) {
+      double acc[2][2][2];
 #pragma unroll
-        for (int a = 0; a < 2; ++a)
+      for (int a = 0; a < 2; ++a)
 #pragma unroll
-          for (int b = 0; b < 4; ++b) { acc[a][b][0] = 0.0; acc[a][b][1] = 0.0; }
-        const int row0 = sl * 16;
-        for (int kk = 0; kk < kp; kk += 4) {
-          double af[2], bf[4];
+        for (int b = 0; b < 2; ++b) { acc[a][b][0] = 0.0; acc[a][b][1] = 0.0; }
+      const double* const pw = Wm + (sl * 16 + lr) * ldw + lc;
+      const double* const px = SIDE == 0 ? Xs + (half * 16 + lr) * ldx + lc : Xs + lc * ldx + half * 16 + lr;
+      // left: rows sl*16.. of W^T times columns half*16.. of the tile;
+      // right: rows half*16.. of the tile times columns sl*16.. of W
+      for (int kk = 0; kk < kp; kk += 4) {
+        double wf[2], xf[2];
 #pragma unroll
-          for (int a = 0; a < 2; ++a) af[a] = Wm[(row0 + a * 8 + lr) * ldw + kk + lc];
-#pragma unroll
-          for (int b = 0; b < 4; ++b) bf[b] = Xs[(kk + lc) * 36 + b * 8 + lr];
-#pragma unroll
-          for (int a = 0; a < 2; ++a)
-#pragma unroll
-            for (int b = 0; b < 4; ++b) dmma_8x8x4(acc[a][b][0], acc[a][b][1], af[a], bf[b]);
+        for (int a = 0; a < 2; ++a) {
+          wf[a] = pw[a * 8 * ldw + kk];
+          xf[a] = SIDE == 0 ? px[a * 8 * ldx + kk] : px[kk * ldx + a * 8];
         }
 #pragma unroll
         for (int a = 0; a < 2; ++a)
-#pragma unroll
-          for (int b = 0; b < 4; ++b)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              const int i = row0 + a * 8 + lr;
-              const int j = b * 8 + lc * 2 + e;
-              if (i < k && j < ncol) J.M[(J.r0 + i) + (int64_t)(c0 + j) * J.ld] = acc[a][b][e];
-            }
-      }
-    } else {
-      const int ldx = kpmax + 4;
-      const int r0 = J.r0 + tile * kUpdTile;
-      const int nrow = min(kUpdTile, J.r0 + J.len - r0);
-      for (int sl = warp; sl < nslice; sl += (int)(blockDim.x >> 5)) {
-        double acc[4][2][2];
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int b = 0; b < 2; ++b) { acc[a][b][0] = 0.0; acc[a][b][1] = 0.0; }
-        const int col0 = sl * 16;
-        for (int kk = 0; kk < kp; kk += 4) {
-          double af[4], bf[2];
-#pragma unroll
-          for (int a = 0; a < 4; ++a) af[a] = Xs[(a * 8 + lr) * ldx + kk + lc];
-#pragma unroll
-          for (int b = 0; b < 2; ++b) bf[b] = Wm[(kk + lc) * ldw + col0 + b * 8 + lr];
-#pragma unroll
-          for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int b = 0; b < 2; ++b) dmma_8x8x4(acc[a][b][0], acc[a][b][1], af[a], bf[b]);
-        }
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
 #pragma unroll
           for (int b = 0; b < 2; ++b)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              const int i = a * 8 + lr;
-              const int j = col0 + b * 8 + lc * 2 + e;
-              if (i < nrow && j < k) J.M[(r0 + i) + (int64_t)(J.c0 + j) * J.ld] = acc[a][b][e];
-            }
+            dmma_8x8x4(acc[a][b][0], acc[a][b][1], SIDE == 0 ? wf[a] : xf[a], SIDE == 0 ? xf[b] : wf[b]);
       }
+      const int c0 = J.c0 + tile * kUpdTile, r0 = J.r0 + tile * kUpdTile;
+      const int lim = SIDE == 0 ? min(kUpdTile, J.c0 + J.len - c0) : min(kUpdTile, J.r0 + J.len - r0);
+#pragma unroll
+      for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            if (SIDE == 0) {
+              const int i = sl * 16 + a * 8 + lr, j = half * 16 + b * 8 + lc * 2 + e;
+              if (i < k && j < lim) J.M[(J.r0 + i) + (int64_t)(c0 + j) * J.ld] = acc[a][b][e];
+            } else {
+              const int i = half * 16 + a * 8 + lr, j = sl * 16 + b * 8 + lc * 2 + e;
+              if (i < lim && j < k) J.M[(r0 + i) + (int64_t)(J.c0 + j) * J.ld] = acc[a][b][e];
+            }
+          }
     }
     __syncthreads();  // this buffer and the factor are free again
   }
