@@ -54,7 +54,7 @@ __device__ __forceinline__ double block_sum(double v, double* red) {
 
 }  // namespace
 
-__global__ void __launch_bounds__(kBatchThreads) k_batch_qz(int count, const int* __restrict__ order,
+__global__ void __launch_bounds__(kBatchThreads, 1) k_batch_qz(int count, const int* __restrict__ order,
                                                             const int* __restrict__ nsz,
                                                             const int64_t* __restrict__ moff,
                                                             const int64_t* __restrict__ eoff, double* H, double* T,

@@ -250,58 +250,44 @@ struct RoleCore {
     double* rp = (isT ? Tb : Hb) + f + (lane < 7 ? rr : 0) + f * ld;
     double* dh = Hb + f + f * ld;  // H(s, s)
     double* dt = Tb + f + f * ld;  // T(s, s)
+    // The left rotations of the first step; each step forms the next one's as
+    // soon as it has the bulge column, ahead of its own stores.  (The added
+    // constant stands in for a1 = a2 = 0 and is below 1e-24 of the largest
+    // entry in range.)
+    double c1, s1, c2, s2, beta, q23, q;
+    auto left = [&]() {
+      const double a1t = a1 + 1e-145;
+      q23 = a1t * a1t + a2 * a2;
+      q = a0 * a0 + q23;
+      const double v1 = role_rsqrt(q23), v2 = role_rsqrt(q);
+      c1 = a1t * v1; s1 = a2 * v1; c2 = a0 * v2; s2 = (q23 * v1) * v2; beta = q * v2;
+    };
+    left();
     for (int s = f; s < l - 1; ++s, rp += diag, dh += diag, dt += diag) {
       const int c = s + lane;
       const bool has = c < n, two = s + 32 < n, has2 = c + 32 < n;
-      // (lanes without a column read the block's first one)
+      // a lane per column: rows s..s+2 of H and T (lanes without a column
+      // read the block's first one); column s+2 of T for all
       const int o1 = has ? lane * ld : 0, o2 = has2 ? o1 + far : 0;
-      const double h0 = dh[o1], h1 = dh[o1 + 1], h2 = dh[o1 + 2], u0 = dt[o1], u1 = dt[o1 + 1], u2 = dt[o1 + 2];
+      double h0 = dh[o1], h1 = dh[o1 + 1], h2 = dh[o1 + 2], u0 = dt[o1], u1 = dt[o1 + 1], u2 = dt[o1 + 2];
+      const double t02 = dt[2 * ld], t12 = dt[2 * ld + 1], t22 = dt[2 * ld + 2];
       double p0 = 0.0, p1 = 0.0, p2 = 0.0, w0 = 0.0, w1 = 0.0, w2 = 0.0;
       if (two) {
         p0 = dh[o2]; p1 = dh[o2 + 1]; p2 = dh[o2 + 2];
         w0 = dt[o2]; w1 = dt[o2 + 1]; w2 = dt[o2 + 2];
       }
-      const double t02 = dt[2 * ld], t12 = dt[2 * ld + 1], t22 = dt[2 * ld + 2];
-      // the previous step is complete: post it (its stores are long done, so
-      // the release waits for nothing)
-      role_post(lane == 0, &rb->ready, g);
-      // left rotations (the added constant stands in for a1 = a2 = 0 and is
-      // below 1e-24 of the largest entry in range)
-      const double a1t = a1 + 1e-145;
-      const double q23 = a1t * a1t + a2 * a2, q = a0 * a0 + q23;
-      const double v1 = role_rsqrt(q23), v2 = role_rsqrt(q);
-      double c1 = a1t * v1, s1 = a2 * v1, c2 = a0 * v2, s2 = (q23 * v1) * v2, beta = q * v2;
-      // rows s+1, s+2 of T's block after them
-      double y0 = -s2 * t00, x1 = -s1 * t11, y1 = c2 * (c1 * t11) - s2 * t01;
-      double x2 = c1 * t22 - s1 * t12, y2 = c2 * (c1 * t12 + s1 * t22) - s2 * t02;
-      double e0 = h0, e1 = h1, e2 = h2, d0 = u0, d1 = u1, d2 = u2;
-      role_apply_left(c1, s1, c2, s2, e0, e1, e2);
-      role_apply_left(c1, s1, c2, s2, d0, d1, d2);
-      // right rotations
-      const double qb = x1 * x1 + x2 * x2, dd = x2 * y1 - x1 * y2, qc = dd * dd + (y0 * y0) * qb;
-      const double vb = role_rsqrt(qb), vc = role_rsqrt(qc);
-      double cb = x2 * vb, sb = x1 * vb, cc = dd * vc, sc = (y0 * (qb * vb)) * vc;
-      if (!(role_in_range(q) && q23 > 0.5 * kRoleTiny && role_in_range(qb) && role_in_range(qc))) {
+      if (!(role_in_range(q) && q23 > 0.5 * kRoleTiny)) {
         const RoleRot o = role_left_scaled(a0, a1, a2);
         c1 = o.c1; s1 = o.s1; c2 = o.c2; s2 = o.s2; beta = o.r;
-        y0 = -s2 * t00; x1 = -s1 * t11; y1 = c2 * (c1 * t11) - s2 * t01;
-        x2 = c1 * t22 - s1 * t12; y2 = c2 * (c1 * t12 + s1 * t22) - s2 * t02;
-        const RoleRot z = role_right_scaled(x1, x2, y0, y1, y2);
-        cb = z.c1; sb = z.s1; cc = z.c2; sc = z.s2;
-        e0 = h0; e1 = h1; e2 = h2; d0 = u0; d1 = u1; d2 = u2;
-        role_apply_left(c1, s1, c2, s2, e0, e1, e2);
-        role_apply_left(c1, s1, c2, s2, d0, d1, d2);
       }
       if (!slot_free()) return false;
+      role_apply_left(c1, s1, c2, s2, h0, h1, h2);
+      role_apply_left(c1, s1, c2, s2, u0, u1, u2);
+      const unsigned ar = role_sm(rb->ring[g & (kRoleRing - 1)]);
       __syncwarp();
-      {
-        const unsigned ah = role_sm(dh + o1), at = role_sm(dt + o1), ar = role_sm(rb->ring[g & (kRoleRing - 1)]);
-        role_put3(has, ah, 8, e0, e1, e2);
-        role_put3(has, at, 8, d0, d1, d2);
-        role_put(s > f && lane < 3, role_sm(dh + (lane - ld)), lane == 0 ? beta : 0.0);
-        role_put8(lane == 0, ar, c1, s1, c2, s2, cb, sb, cc, sc);
-        role_put_int2(lane == 0, ar + 64, s, 3);
-      }
+      role_put3(has, role_sm(dh + o1), 8, h0, h1, h2);
+      role_put3(has, role_sm(dt + o1), 8, u0, u1, u2);
+      role_put(s > f && lane < 3, role_sm(dh + (lane - ld)), lane == 0 ? beta : 0.0);
       __syncwarp();
       // rows s+1..s+3 of H for all (row l + 1 is outside the block), and the
       // lane's row
@@ -309,42 +295,53 @@ struct RoleCore {
       const bool in3 = s + 3 <= l, rowok = isT ? lane < 7 : s + lane <= l;
       const double g10 = hr[0], g11 = hr[ld], g12 = hr[2 * ld], g20 = hr[1], g21 = hr[1 + ld], g22 = hr[1 + 2 * ld];
       const double q30 = hr[2], q31 = hr[2 + ld], q32 = hr[2 + 2 * ld];  // past the window's last row: not used
-      const double g30 = in3 ? q30 : 0.0, g31 = in3 ? q31 : 0.0, g32 = in3 ? q32 : 0.0;
       double r0 = rp[0], r1 = rp[ld], r2 = rp[2 * ld];
+      // rows s+1, s+2 of T's block after the left rotations, and the right ones
+      const double y0 = -s2 * t00, x1 = -s1 * t11, y1 = c2 * (c1 * t11) - s2 * t01;
+      const double x2 = c1 * t22 - s1 * t12, y2 = c2 * (c1 * t12 + s1 * t22) - s2 * t02;
+      const double qb = x1 * x1 + x2 * x2, dd = x2 * y1 - x1 * y2, qc = dd * dd + (y0 * y0) * qb;
+      const double vb = role_rsqrt(qb), vc = role_rsqrt(qc);
+      double cb = x2 * vb, sb = x1 * vb, cc = dd * vc, sc = (y0 * (qb * vb)) * vc;
+      if (!(role_in_range(qb) && role_in_range(qc))) {
+        const RoleRot z = role_right_scaled(x1, x2, y0, y1, y2);
+        cb = z.c1; sb = z.s1; cc = z.c2; sc = z.s2;
+      }
+      role_put8(lane == 0, ar, c1, s1, c2, s2, cb, sb, cc, sc);
+      role_put_int2(lane == 0, ar + 64, s, 3);
       if (two) {
         role_apply_left(c1, s1, c2, s2, p0, p1, p2);
         role_apply_left(c1, s1, c2, s2, w0, w1, w2);
+        role_put3(has2, role_sm(dh + o2), 8, p0, p1, p2);
+        role_put3(has2, role_sm(dt + o2), 8, w0, w1, w2);
+        // columns from s + 64 on
+        for (int k = c + 64; k < n; k += 32) {
+          double* const hq = Hb + s + k * ld;
+          double* const tq = Tb + s + k * ld;
+          double b0 = hq[0], b1 = hq[1], b2 = hq[2], f0 = tq[0], f1 = tq[1], f2 = tq[2];
+          role_apply_left(c1, s1, c2, s2, b0, b1, b2);
+          role_apply_left(c1, s1, c2, s2, f0, f1, f2);
+          hq[0] = b0; hq[1] = b1; hq[2] = b2;
+          tq[0] = f0; tq[1] = f1; tq[2] = f2;
+        }
       }
-      // the next step's bulge column and block of T
+      // the next step's bulge column, block of T and left rotations
+      a0 = cc * g10 - sc * (cb * g11 - sb * g12);
+      a1 = cc * g20 - sc * (cb * g21 - sb * g22);
+      a2 = cc * q30 - sc * (cb * q31 - sb * q32);
+      a2 = in3 ? a2 : 0.0;
+      left();
       t00 = cc * (cb * y1 - sb * y2) + sc * y0;
       t01 = cb * y2 + sb * y1;
       t11 = cb * x2 + sb * x1;
-      a0 = cc * g10 - sc * (cb * g11 - sb * g12);
-      a1 = cc * g20 - sc * (cb * g21 - sb * g22);
-      a2 = cc * g30 - sc * (cb * g31 - sb * g32);
       role_apply_right(cb, sb, cc, sc, r0, r1, r2);
       r0 = isT && rr >= 1 ? 0.0 : r0;
       r1 = isT && rr >= 2 ? 0.0 : r1;
       __syncwarp();
       role_put3(rowok, role_sm(rp), 8 * ld, r0, r1, r2);
-      if (two) {
-        role_put3(has2, role_sm(dh + o2), 8, p0, p1, p2);
-        role_put3(has2, role_sm(dt + o2), 8, w0, w1, w2);
-      }
-      // columns from s + 64 on
-      for (int k = c + 64; k < n; k += 32) {
-        double* const hq = Hb + s + k * ld;
-        double* const tq = Tb + s + k * ld;
-        double b0 = hq[0], b1 = hq[1], b2 = hq[2], f0 = tq[0], f1 = tq[1], f2 = tq[2];
-        role_apply_left(c1, s1, c2, s2, b0, b1, b2);
-        role_apply_left(c1, s1, c2, s2, f0, f1, f2);
-        hq[0] = b0; hq[1] = b1; hq[2] = b2;
-        tq[0] = f0; tq[1] = f1; tq[2] = f2;
-      }
       ++g;
       __syncwarp();
+      role_post(lane == 0, &rb->ready, g);
     }
-    __syncwarp();
     // final 2x2 step at rows and columns l-1, l
     const int s = l - 1;
     double c, sn, r;
