@@ -122,8 +122,10 @@ __global__ void __launch_bounds__(kThreads) k_aed_win(double* H, double* T, int6
     x.stamp(0);
     const int qz = cta_role_qz(x, w, maxit, (RoleBuf*)scr);
     if (qz == 0) cta_std_all(x, w, sd + 64);
-    cta_aed_deflate(x, w, s, shifts, shifts + n, shifts + 2 * n, qz, nskip, swapfail != 0,
-                    [&](int m) { return cta_role_hessred(x, w, m, (RoleBuf*)scr); });
+    cta_aed_deflate(
+        x, w, s, shifts, shifts + n, shifts + 2 * n, qz,
+        [&]() { return cta_role_spike(x, w, s, nskip, swapfail != 0, (RoleBuf*)scr); },
+        [&](int m) { return cta_role_hessred(x, w, m, (RoleBuf*)scr); });
   } else {
     cta_aed(x, w, s, shifts, shifts + n, shifts + 2 * n, maxit, nskip, swapfail != 0, ms ? scr : nullptr);
   }

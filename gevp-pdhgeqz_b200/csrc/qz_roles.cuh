@@ -613,6 +613,197 @@ __device__ int cta_role_qz(X& x, WinState& w, int maxit, RoleBuf* rb) {
 }
 
 // ---------------------------------------------------------------------------
+// Several block swaps at once (disjoint blocks): a thread forms each, the
+// block applies their factors.
+// ---------------------------------------------------------------------------
+constexpr int kRoleSwap = 64;  // a swap's record: Q, Z, S2, T2 (16 each)
+// one swap of blocks of sizes N1, N2 at window row j, by one thread, to rec
+template <int N1, int N2>
+__device__ __forceinline__ bool role_swap(double* S, double* T, int ld, int j, const Tol& tol, double* rec) {
+  constexpr int M = N1 + N2;
+  const MatV hb{S + j + j * ld, ld}, tb{T + j + j * ld, ld};
+  double S2[M * M], T2[M * M], Qs[M * M], Zs[M * M];
+  int res;
+  if constexpr (N1 == 1 && N2 == 1)
+    // two rotations; the Sylvester path where they fail the stability test
+    res = swap_compute11(hb, tb, S2, T2, Qs, Zs, tol.ulp, tol.smlnum)
+              ? 1
+              : swap_compute_try<1, 1>(hb, tb, S2, T2, Qs, Zs, tol.ulp, tol.smlnum);
+  else
+    res = swap_compute_try<N1, N2>(hb, tb, S2, T2, Qs, Zs, tol.ulp, tol.smlnum);
+  if (res > 0) {
+#pragma unroll
+    for (int i = 0; i < M * M; ++i) { rec[i] = Qs[i]; rec[16 + i] = Zs[i]; rec[32 + i] = S2[i]; rec[48 + i] = T2[i]; }
+    return true;
+  }
+  return res < 0 && swap_retry<N1, N2>(hb, tb, rec + 32, rec + 48, rec, rec + 16, tol.ulp, tol.smlnum);
+}
+
+// y = F^T x (rows) or x F (columns) for the M entries at p, p + st, ..: the
+// same sums, F = Q or Z
+template <int M>
+__device__ __forceinline__ void role_line(const double* f, double* p, int st) {
+  double x[M];
+#pragma unroll
+  for (int i = 0; i < M; ++i) x[i] = p[i * st];
+#pragma unroll
+  for (int c = 0; c < M; ++c) {
+    double a = 0.0;
+#pragma unroll
+    for (int k = 0; k < M; ++k) a += x[k] * f[k + M * c];
+    p[c * st] = a;
+  }
+}
+__device__ __forceinline__ void role_line_any(int m, const double* f, double* p, int st) {
+  if (m == 2) role_line<2>(f, p, st);
+  else if (m == 3) role_line<3>(f, p, st);
+  else role_line<4>(f, p, st);
+}
+
+
+// The swaps sw[0..np) (row | size of the first block << 8 | of the second
+// << 12) of one window, by all threads of a block: recs holds np records,
+// good[k] tells whether swap k was applied.  Ends with a barrier.
+template <class X>
+__device__ void cta_role_swaps(X& x, const WinState& w, const int* sw, int np, double* recs, int* good) {
+  const int tid = x.tid, warp = tid >> 5, lane = tid & 31, nw = x.nt >> 5, ld = w.H.ld, n = w.n;
+  double *const Hs = w.H.p, *const Ts = w.T.p, *const Us = w.Q.p, *const Vs = w.Z.p;
+  // a thread per swap, the four kinds on four warps
+  if (warp < 4)
+    for (int k = lane; k < np; k += 32) {
+      const int e = sw[k], j = e & 255, n1 = (e >> 8) & 15, n2 = e >> 12;
+      if (2 * (n1 - 1) + n2 - 1 != warp) continue;
+      double* const rec = recs + k * kRoleSwap;
+      if (warp == 0) good[k] = role_swap<1, 1>(Hs, Ts, ld, j, w.tol, rec);
+      else if (warp == 1) good[k] = role_swap<1, 2>(Hs, Ts, ld, j, w.tol, rec);
+      else if (warp == 2) good[k] = role_swap<2, 1>(Hs, Ts, ld, j, w.tol, rec);
+      else good[k] = role_swap<2, 2>(Hs, Ts, ld, j, w.tol, rec);
+    }
+  x.sync();
+  // left factors: rows of H, T right of the block; columns of Q
+  for (int k = warp; k < np; k += nw) {
+    if (!good[k]) continue;
+    const int e = sw[k], j = e & 255, m = ((e >> 8) & 15) + (e >> 12);
+    const double* const rec = recs + k * kRoleSwap;
+    for (int c = j + m + lane; c < n; c += 32) {
+      role_line_any(m, rec, Hs + j + c * ld, 1);
+      role_line_any(m, rec, Ts + j + c * ld, 1);
+    }
+    for (int i = lane; i < n; i += 32) role_line_any(m, rec, Us + i + j * ld, ld);
+  }
+  x.sync();
+  // right factors: columns of H, T above the block; columns of Z; the block
+  for (int k = warp; k < np; k += nw) {
+    if (!good[k]) continue;
+    const int e = sw[k], j = e & 255, m = ((e >> 8) & 15) + (e >> 12);
+    const double* const rec = recs + k * kRoleSwap;
+    for (int i = lane; i < j; i += 32) {
+      role_line_any(m, rec + 16, Hs + i + j * ld, ld);
+      role_line_any(m, rec + 16, Ts + i + j * ld, ld);
+    }
+    for (int i = lane; i < n; i += 32) role_line_any(m, rec + 16, Vs + i + j * ld, ld);
+    if (lane < m * m) {
+      Hs[j + lane % m + (j + lane / m) * ld] = rec[32 + lane];
+      Ts[j + lane % m + (j + lane / m) * ld] = rec[48 + lane];
+    }
+  }
+  x.sync();
+}
+
+// ---------------------------------------------------------------------------
+// Spike test with reordering (the loop of cta_aed_deflate) with the moves of
+// undeflatable blocks overlapped.  A move's first swap settles the block that
+// is tested next, so the next test and the next move start a round later and
+// follow the earlier move up the window, two blocks behind; a round forms the
+// swaps of all moves under way at once.  The same tests on the same blocks in
+// the same order as one move after another; returns the last undeflated row.
+// A rejected swap ends the test with the moves where they are.
+// Bound: a swap's serial computation per round; a window of 48 takes about 26
+// rounds instead of 88 swaps in sequence when the test stops after four
+// undeflatable blocks.
+// ---------------------------------------------------------------------------
+constexpr int kRoleMoves = kRoleDoubles / kRoleSwap;  // records in the role buffer
+template <class X>
+__device__ int cta_role_spike(X& x, WinState& w, double s, int nskip, bool swapfail, RoleBuf* rb) {
+  const int n = w.n;
+  double* const recs = (double*)rb;
+  int* const sw = x.si + 16;              // swaps of the round
+  int* const good = sw + kRoleMoves;
+  int* const ctl = good + kRoleMoves;     // swaps, last row
+  // thread 0's: moves under way, in order
+  int pos[kRoleMoves], size[kRoleMoves], goal[kRoleMoves], act = 0;
+  int who[kRoleMoves];
+  int kb = n - 1, ilst = 0, fails = 0;
+  bool stop = false;
+  for (;;) {
+    int np = 0;
+    if (x.tid == 0) {
+      // settled blocks at the bottom
+      while (!stop && act < kRoleMoves) {
+        if (kb < ilst || (nskip > 0 && fails >= nskip)) { stop = true; break; }
+        const int free0 = act ? pos[act - 1] + size[act - 1] : 0;
+        if (kb < free0) break;
+        const bool bulge = (kb > ilst) && (w.H(kb, kb - 1) != 0.0);
+        const int nb = bulge ? 2 : 1, at = kb - nb + 1;
+        if (at < free0) break;
+        bool dfl;
+        if (!bulge) {
+          const double temp = fabs(s) + fabs(w.H(kb, kb));
+          dfl = fabs(s * w.Q(0, kb)) <= dmax(w.tol.ulp * temp, w.tol.smlnum);
+        } else {
+          const double h11 = w.H(kb - 1, kb - 1), h21 = w.H(kb, kb - 1), h12 = w.H(kb - 1, kb), h22 = w.H(kb, kb);
+          double rtdet;
+          if (h11 == 0.0 && h21 == 0.0) rtdet = 0.0;
+          else if (fabs(h11) >= fabs(h21)) rtdet = sqrt(fabs(h11)) * sqrt(fabs(h22 - (h21 / h11) * h12));
+          else rtdet = sqrt(fabs(h21)) * sqrt(fabs(h12 - (h11 / h21) * h22));
+          const double temp = fabs(s) + rtdet;
+          dfl = dmax(fabs(s * w.Q(0, kb)), fabs(s * w.Q(0, kb - 1))) <= dmax(w.tol.ulp * temp, w.tol.smlnum);
+        }
+        if (dfl) { kb -= nb; fails = 0; continue; }
+        if (swapfail) { stop = true; act = 0; break; }
+        if (at > ilst) {
+          pos[act] = at;
+          size[act] = nb;
+          goal[act] = ilst;
+          ++act;
+        }
+        ilst += nb;
+        ++fails;
+      }
+      for (int i = 0; i < act; ++i) {
+        const int nbn = (pos[i] - 2 >= goal[i] && w.H(pos[i] - 1, pos[i] - 2) != 0.0) ? 2 : 1, lo = pos[i] - nbn;
+        if (i > 0 && lo < pos[i - 1] + size[i - 1]) continue;
+        sw[np] = lo | nbn << 8 | size[i] << 12;
+        who[np++] = i;
+      }
+      ctl[0] = np;
+      ctl[1] = kb;
+    }
+    x.sync();
+    np = ctl[0];
+    if (np == 0) break;
+    cta_role_swaps(x, w, sw, np, recs, good);
+    if (x.tid == 0) {
+      for (int k = 0; k < np; ++k) {
+        x.count(1);
+        const int i = who[k];
+        if (!good[k]) { stop = true; act = 0; break; }
+        pos[i] = sw[k] & 255;
+        // the moved block must keep its size (a complex pair stays 2x2)
+        if (size[i] == 2 && w.H(pos[i] + 1, pos[i]) == 0.0) { stop = true; act = 0; break; }
+      }
+      int keep = 0;
+      for (int i = 0; i < act; ++i)
+        if (pos[i] > goal[i]) { pos[keep] = pos[i]; size[keep] = size[i]; goal[keep] = goal[i]; ++keep; }
+      act = keep;
+    }
+  }
+  kb = ctl[1];
+  x.sync();
+  return kb;
+}
+
+// ---------------------------------------------------------------------------
 // Hessenberg-triangular re-reduction of the leading m x m block (the job of
 // cta_hessred, the same rotations up to signs) by kRoleThreads threads.
 //

@@ -310,28 +310,12 @@ QZ_HD void cta_hessred(X& x, WinState& w, int m) {
   }
 }
 
-// The part after the window QZ, whose status is info (0: w is in generalized
-// Schur form with standardised blocks).  hessred(m) re-reduces the leading
-// m x m block; false: it failed, and the window with it.
-template <class X, class HR>
-QZ_HD void cta_aed_deflate(X& x, WinState& w, double s, double* sr, double* si_, double* sb, int info, int nskip,
-                           bool swapfail, const HR& hessred) {
-  int n = w.n;
-  x.stamp(1);
-  if (info != 0) {
-    // window QZ did not converge: deflate nothing, hand the diagonal
-    // ratios of the (equivalent) partly reduced window over as shifts
-    // (qzearly.f:237-248); the caller discards the window itself
-    if (x.tid == 0) {
-      for (int i = 0; i < n; ++i) { sr[i] = w.H(i, i); si_[i] = 0.0; sb[i] = w.T(i, i); }
-      x.si[8] = n; x.si[9] = info; x.si[10] = 0;
-    }
-    x.sync();
-    return;
-  }
-  // ---- spike test with reordering (qzearly.f:253-365) ----
+// Spike test with reordering, one undeflatable block moved up after another:
+// the last undeflated row.
+template <class X>
+QZ_HD int cta_aed_spike(X& x, WinState& w, double s, int nskip, bool swapfail) {
+  const int n = w.n;
   int kb = n - 1, ilst = 0;
-  bool failed = false;
   int fails = 0;  // consecutive undeflatable blocks
   while (kb >= ilst) {
     // optional early stop: after nskip consecutive undeflatable blocks the
@@ -358,12 +342,36 @@ QZ_HD void cta_aed_deflate(X& x, WinState& w, double s, double* sr, double* si_,
     } else {
       // a rejected swap ends the test: the window is re-reduced with the
       // deflations found so far (qzearly.f:321-326); swapfail forces it
-      if (swapfail || !cta_move_block(x, w, kb - nb + 1, nb, ilst, false)) { failed = true; break; }
+      if (swapfail || !cta_move_block(x, w, kb - nb + 1, nb, ilst, false)) break;
       ilst += nb;
       ++fails;
     }
   }
-  (void)failed;
+  return kb;
+}
+
+// The part after the window QZ, whose status is info (0: w is in generalized
+// Schur form with standardised blocks).  spike() is the spike test with
+// reordering and returns the last undeflated row; hessred(m) re-reduces the
+// leading m x m block; false: it failed, and the window with it.
+template <class X, class SP, class HR>
+QZ_HD void cta_aed_deflate(X& x, WinState& w, double s, double* sr, double* si_, double* sb, int info,
+                           const SP& spike, const HR& hessred) {
+  int n = w.n;
+  x.stamp(1);
+  if (info != 0) {
+    // window QZ did not converge: deflate nothing, hand the diagonal
+    // ratios of the (equivalent) partly reduced window over as shifts
+    // (qzearly.f:237-248); the caller discards the window itself
+    if (x.tid == 0) {
+      for (int i = 0; i < n; ++i) { sr[i] = w.H(i, i); si_[i] = 0.0; sb[i] = w.T(i, i); }
+      x.si[8] = n; x.si[9] = info; x.si[10] = 0;
+    }
+    x.sync();
+    return;
+  }
+  // ---- spike test with reordering (qzearly.f:253-365) ----
+  const int kb = spike();
   // the swaps left the 2x2 blocks they touched general: standardise every
   // block of the window at once (T upper triangular again, complex pairs
   // with a positive diagonal block of T)
@@ -543,10 +551,12 @@ QZ_HD void cta_aed(X& x, WinState& w, double s, double* sr, double* si_, double*
                    bool swapfail = false, double* msscr = nullptr) {
   x.stamp(0);
   const int info = msscr ? cta_small_qz_ms(x, w, maxit, msscr) : cta_small_qz(x, w, maxit);
-  cta_aed_deflate(x, w, s, sr, si_, sb, info, nskip, swapfail, [&](int m) {
-    cta_hessred(x, w, m);
-    return true;
-  });
+  cta_aed_deflate(
+      x, w, s, sr, si_, sb, info, [&]() { return cta_aed_spike(x, w, s, nskip, swapfail); },
+      [&](int m) {
+        cta_hessred(x, w, m);
+        return true;
+      });
 }
 
 }  // namespace qz

@@ -66,53 +66,10 @@ struct ReoExec {
 
 // S, T, U, V of the window, Q, Z, S2, T2 (16 each) of a round's swaps (the
 // standardisation's 3n doubles reuse them), their status
-constexpr int kReoRec = 64;
+constexpr int kReoRec = kRoleSwap;
 size_t reo_smem(int wk) {
   return ((size_t)4 * wk * smem_ld(wk) + (size_t)(wk / 2 + 1) * kReoRec + 3 * wk) * sizeof(double) +
          (kReoPairs + 8) * sizeof(int);
-}
-
-// one swap of blocks of sizes N1, N2 at window row j, by one thread, to rec
-template <int N1, int N2>
-__device__ __forceinline__ bool reo_swap(double* S, double* T, int ld, int j, const Tol& tol, double* rec) {
-  constexpr int M = N1 + N2;
-  const MatV hb{S + j + j * ld, ld}, tb{T + j + j * ld, ld};
-  double S2[M * M], T2[M * M], Qs[M * M], Zs[M * M];
-  int res;
-  if constexpr (N1 == 1 && N2 == 1)
-    // two rotations; the Sylvester path where they fail the stability test
-    res = swap_compute11(hb, tb, S2, T2, Qs, Zs, tol.ulp, tol.smlnum)
-              ? 1
-              : swap_compute_try<1, 1>(hb, tb, S2, T2, Qs, Zs, tol.ulp, tol.smlnum);
-  else
-    res = swap_compute_try<N1, N2>(hb, tb, S2, T2, Qs, Zs, tol.ulp, tol.smlnum);
-  if (res > 0) {
-#pragma unroll
-    for (int i = 0; i < M * M; ++i) { rec[i] = Qs[i]; rec[16 + i] = Zs[i]; rec[32 + i] = S2[i]; rec[48 + i] = T2[i]; }
-    return true;
-  }
-  return res < 0 && swap_retry<N1, N2>(hb, tb, rec + 32, rec + 48, rec, rec + 16, tol.ulp, tol.smlnum);
-}
-
-// y = F^T x (rows) or x F (columns) for the M entries at p, p + st, ..: the
-// same sums, F = Q or Z
-template <int M>
-__device__ __forceinline__ void reo_line(const double* f, double* p, int st) {
-  double x[M];
-#pragma unroll
-  for (int i = 0; i < M; ++i) x[i] = p[i * st];
-#pragma unroll
-  for (int c = 0; c < M; ++c) {
-    double a = 0.0;
-#pragma unroll
-    for (int k = 0; k < M; ++k) a += x[k] * f[k + M * c];
-    p[c * st] = a;
-  }
-}
-__device__ __forceinline__ void reo_line_any(int m, const double* f, double* p, int st) {
-  if (m == 2) reo_line<2>(f, p, st);
-  else if (m == 3) reo_line<3>(f, p, st);
-  else reo_line<4>(f, p, st);
 }
 
 // One window per CTA; status[1] is set when a swap is rejected.  A 2x2 block
@@ -148,53 +105,6 @@ __global__ void __launch_bounds__(kReoThreads) k_reorder_win(double* S, int64_t 
     }
   __syncthreads();
   if (!skip) {
-    for (int r = 0; r < W.rounds; ++r) {
-      const int s0 = rounds[W.r0 + r], np = rounds[W.r0 + r + 1] - s0;
-      // a thread per swap, the four kinds on four warps
-      if (warp < 4)
-        for (int k = lane; k < np; k += 32) {
-          const int sw = swaps[s0 + k], j = sw & 255, n1 = (sw >> 8) & 15, n2 = sw >> 12;
-          if (2 * (n1 - 1) + n2 - 1 != warp) continue;
-          double* const rec = recs + k * kReoRec;
-          bool ok;
-          if (warp == 0) ok = reo_swap<1, 1>(Hs, Ts, ld, j, tol, rec);
-          else if (warp == 1) ok = reo_swap<1, 2>(Hs, Ts, ld, j, tol, rec);
-          else if (warp == 2) ok = reo_swap<2, 1>(Hs, Ts, ld, j, tol, rec);
-          else ok = reo_swap<2, 2>(Hs, Ts, ld, j, tol, rec);
-          good[k] = ok;
-          if (!ok) *bad = 1;
-        }
-      __syncthreads();
-      // left factors: rows of S, T right of the block; columns of U
-      for (int k = warp; k < np; k += nw) {
-        if (!good[k]) continue;
-        const int sw = swaps[s0 + k], j = sw & 255, m = ((sw >> 8) & 15) + (sw >> 12);
-        const double* const rec = recs + k * kReoRec;
-        for (int c = j + m + lane; c < wk; c += 32) {
-          reo_line_any(m, rec, Hs + j + c * ld, 1);
-          reo_line_any(m, rec, Ts + j + c * ld, 1);
-        }
-        for (int i = lane; i < wk; i += 32) reo_line_any(m, rec, Us + i + j * ld, ld);
-      }
-      __syncthreads();
-      // right factors: columns of S, T above the block; columns of V; the block
-      for (int k = warp; k < np; k += nw) {
-        if (!good[k]) continue;
-        const int sw = swaps[s0 + k], j = sw & 255, m = ((sw >> 8) & 15) + (sw >> 12);
-        const double* const rec = recs + k * kReoRec;
-        for (int i = lane; i < j; i += 32) {
-          reo_line_any(m, rec + 16, Hs + i + j * ld, ld);
-          reo_line_any(m, rec + 16, Ts + i + j * ld, ld);
-        }
-        for (int i = lane; i < wk; i += 32) reo_line_any(m, rec + 16, Vs + i + j * ld, ld);
-        if (lane < m * m) {
-          Hs[j + lane % m + (j + lane / m) * ld] = rec[32 + lane];
-          Ts[j + lane % m + (j + lane / m) * ld] = rec[48 + lane];
-        }
-      }
-      __syncthreads();
-      if (*bad) break;
-    }
     ReoExec x{tid, (int)blockDim.x, nullptr, recs};
     WinState w;
     w.n = wk;
@@ -205,6 +115,12 @@ __global__ void __launch_bounds__(kReoThreads) k_reorder_win(double* S, int64_t 
     w.wantq = true;
     w.wantz = true;
     w.tol = tol;
+    for (int r = 0; r < W.rounds && !*bad; ++r) {
+      const int s0 = rounds[W.r0 + r], np = rounds[W.r0 + r + 1] - s0;
+      cta_role_swaps(x, w, swaps + s0, np, recs, good);
+      if (tid < np && !good[tid]) *bad = 1;
+      __syncthreads();
+    }
     cta_std_all(x, w, recs);
     if (tid == 0 && *bad) status[1] = 1;
     for (int j = warp; j < wk; j += nw)
