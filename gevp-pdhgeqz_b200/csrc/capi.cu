@@ -194,20 +194,20 @@ struct GpuBackend {
     if (c->err != cudaSuccess) { out[0] = ifirst; out[1] = 0; out[2] = -1; out[3] = -1; out[4] = 1; return; }
     for (int i = 0; i < 5; ++i) out[i] = c->hinfo[i];
   }
-  // consecutive undeflatable blocks after which the spike test stops
-  // (0: the whole window).  Automatic: the whole window for pencils of
-  // order 6000 and more (measured: -34 % time to Schur at n = 10000 against
-  // stopping after 4), 4 below (-16 % at n = 2000 against the whole window)
-  int aed_early_stop(int nh) const {
-    (void)nh;
+  // Consecutive undeflatable blocks after which the spike test stops (0: the
+  // whole window).  Automatic: the whole window for pencils of order 900 and
+  // more (n=1800: 387 against 410 ms stopping after 4, n=901 145 against
+  // 148), 4 below, where a window's moves cost more than the sweeps they save
+  // (n=700 123 against 130, n=201 30 against 38).
+  int aed_early_stop() const {
     if (c->params.aed_nskip >= 0) return c->params.aed_nskip;
-    return n >= 6000 ? 0 : 4;
+    return n >= 900 ? 0 : 4;
   }
   void aed(int ktop, int kwtop, int kbot, int* info3, double* sh) {
     int nw = kbot - kwtop + 1;
     c->timer.begin(kPhAed, c->stream);
     launch_aed(c->stream, H, T, ld, ktop, kwtop, nw, tol, c->Ua, c->Va, c->shifts, c->dinfo + 4, c->gscratch,
-               c->timer.on ? c->dts : nullptr, (kwtop > ktop) ? aed_early_stop(kbot - ktop + 1) : 0,
+               c->timer.on ? c->dts : nullptr, (kwtop > ktop) ? aed_early_stop() : 0,
                c->params.aed_threads, c->params.aed_swap_fail, c->params.aed_ms);
     c->stats.launches += 1;
     c->stats.aed_launches += 1;

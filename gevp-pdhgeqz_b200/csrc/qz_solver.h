@@ -22,7 +22,7 @@ namespace qz {
 // Tunables (defaults follow the reference's PIPARMQ table where the GPU
 // window limits allow; see piparmq.f:438-535).
 struct SolveParams {
-  int nw_max = 48;       // AED window (one CTA, shared memory; up to 80)
+  int nw_max = 0;        // AED window (one CTA, shared memory; up to 80); 0: table
   int w_chase = 64;      // chase window and bulges per chain: 64 and 8 (a bulge per
                          // chase warp).  A step of the chase kernel costs 2,270
                          // cycles there and 4,340 for 12 bulges in 80 rows, and the
@@ -30,14 +30,14 @@ struct SolveParams {
                          // chase + updates of an n=1800 solve 264 ms at (64, 8),
                          // 381 at (80, 12), 281 at (48, 6), 329 at (32, 4)
   int nmin = 80;         // active blocks this small are solved by one CTA
-  int nibble = -1;       // -1: table (14 in PDHGEQZ1 regime, 335*nh^-0.44 above)
+  int nibble = -1;       // -1: table (nibble_table)
   int ns_max = -1;       // -1: table
   int maxit_factor = 30; // MAXIT = 30*NH
   int chain_max = 8;     // -1: from w_chase
   int verbose = 0;       // progress lines on stderr (B200QZ_VERBOSE=1)
   int aed_nskip = -1;    // AED spike test stops after this many consecutive
                          // undeflatable blocks (0: test the whole window;
-                         // -1: whole window for n >= 6000, else 4)
+                         // -1: whole window for n >= 900, else 4)
   int max_wave = 8;      // chains chased concurrently (one CTA each)
   int stall_limit = 300; // iterations without deflation before giving up
   int aed_threads = 256; // threads of the AED / endgame window kernel (256: a role
@@ -84,9 +84,28 @@ inline int ns_table(int nh) {
   if (nh >= 12000) ns = 512;
   return std::max(2, ns - ns % 2);
 }
+// Share of the window (in %) that an AED has to deflate for the next step to
+// be another AED instead of a sweep.  The reference's 14 up to nh = 6000
+// (piparmq.f:495-496) weighs an AED against its own sweeps; here an AED costs
+// 0.6 (window 24) to 2 ms on one SM and a sweep 0.3 ms at n=200, 2.4 ms at
+// n=1800, so a sweep comes sooner.  Measured with 14 / 40 / 60: n=201 47 / 33 /
+// 38 ms, n=901 226 / 169 / 184, n=1800 482 / 410 / 439, n=4000 - / 1264 / 1328.
 inline int nibble_table(int nh) {
-  if (nh <= 6000) return 14;  // PDHGEQZ1 regime (piparmq.f:495-496)
+  if (nh <= 6000) return 40;
   return std::min(100, (int)std::ceil(335.0 * std::pow((double)nh, -0.44)));
+}
+
+// AED window of a pencil of order nh.  A window costs about nw^2 steps of one
+// SM, a sweep about nh steps of several, so small pencils want small windows.
+// (The order the solve began with: taking the active block's instead, which
+// shrinks, costs 408 ms at n=1800 for 387.)  Measured (ms) with 24 / 32 / 48 / 56: n=201 24.8 / 29.5 / 32.6 / -,
+// n=500 75 / 75 / 96 / -, n=901 155 / 148 / 169 / -, n=1800 - / 497 / 387 /
+// 390, n=4000 - / - / 1264 / 1212.
+inline int nw_table(int nh) {
+  if (nh < 600) return 24;
+  if (nh < 1200) return 32;
+  if (nh < 3000) return 48;
+  return 56;
 }
 
 // Power of two applied to T before the iteration when T's magnitude is far
@@ -221,7 +240,7 @@ int qz_iterate(BK& bk, int n, int ilo, int ihi, const SolveParams& P, SolveStats
   int ifirst = ilo, kbot = ihi;
   int nh0 = ihi - ilo + 1;
   int64_t maxit = (int64_t)P.maxit_factor * std::max(1, nh0);
-  std::vector<double> sh(3 * std::max(P.nw_max, P.nmin) + 8);
+  std::vector<double> sh(3 * std::max(std::max(P.nw_max, 80), P.nmin) + 8);
   std::vector<ShiftPair> pairs;
   std::vector<const WinPlan*> wave;
   int scan_out[5];
@@ -291,7 +310,7 @@ int qz_iterate(BK& bk, int n, int ilo, int ihi, const SolveParams& P, SolveStats
       S.stop_kbot = kbot;
       return done(-2);
     }
-    int nw = std::min(P.nw_max, nh);
+    int nw = std::min(P.nw_max > 0 ? P.nw_max : nw_table(nh0), nh);
     int ns_pol = -1;
     {
       int pnw = 0, pns = 0;
@@ -354,13 +373,16 @@ int qz_iterate(BK& bk, int n, int ilo, int ihi, const SolveParams& P, SolveStats
     int W = P.w_chase;
     int cmax = (P.chain_max > 0) ? P.chain_max : std::max(1, (W - 4) / 6);
     cmax = std::min(cmax, std::max(1, (W - 4) / 3 - 1));
-    // ---- plan every chain's windows (positions do not depend on data) ----
-    int nbig = std::min(cmax, npairs);
+    // ---- plan every chain's windows (positions do not depend on data);
+    // chains of equal length, which advance further per window than the
+    // longest allowed and a short rest ----
+    const int nchain = (npairs + cmax - 1) / cmax;
+    int nbig = (npairs + nchain - 1) / nchain;
     int adv = W - 4 - 3 * (nbig - 1);  // common advance per window
     std::vector<ChainPlan> plans;
-    for (int p0 = 0; p0 < npairs; p0 += cmax) {
+    for (int p0 = 0; p0 < npairs; p0 += nbig) {
       ChainPlan cp;
-      int nb = std::min(cmax, npairs - p0);
+      int nb = std::min(nbig, npairs - p0);
       plan_chain(ktop, kbot, W, nb, pairs.data() + p0, adv, cp);
       plans.push_back(std::move(cp));
       ++S.chains;

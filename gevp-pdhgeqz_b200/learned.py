@@ -40,7 +40,7 @@ TRACES = os.path.join(POLICY_DIR, "traces.npz")
 
 NIN, NHID, NOUT = 64, 128, 2
 NW_MIN, NW_SPAN, NW_MAX = 16, 64, 80
-TABLE_NW = 48  # the solver's fixed AED window (SolveParams::nw_max)
+TABLE_NW = 48  # the fixed AED window the policy is compared with
 GRID_NW = (24, 32, 40, 48, 56, 64, 80)
 GRID_NSF = (0.5, 1.0)
 DECISIONS = (0, 5, 20, 60, 150)  # AED indices at which a trace samples the choice
