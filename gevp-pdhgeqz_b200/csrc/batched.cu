@@ -5,14 +5,18 @@
 // CTA-level kernels as the endgame (PDHGEQZ4 -> KKQZ): every pencil is
 // reduced to generalized Schur form with Q and Z by one CTA.
 //
-// One persistent launch: CTAs pull pencils from an atomic queue ordered by
-// decreasing size (longest-first scheduling), solve a pencil in shared
-// memory when n <= kBatchSmemMax (H, T, Q, Z with an odd leading
-// dimension), in place in global memory otherwise, normalise beta >= 0 and
-// write the eigenvalues.  Pencils in shared memory take the window QZ with
-// a role per warp (qz_roles.cuh: 3.8x the two-barrier sweeps at orders up to
-// 80); the others, and launches with 128 threads, small-bulge multishift
-// sweeps (cta_small_qz_ms).  Per-pencil status words; no host round trip.
+// CTAs pull pencils from an atomic queue ordered by decreasing size
+// (longest-first scheduling).  Two persistent launches: pencils of order up to
+// kBatchSmemMax are solved in shared memory (H, T, Q, Z with an odd leading
+// dimension) by the window QZ with a role per warp (qz_roles.cuh: 600 pencils
+// of order 16..80 in 7.0 ms, 33.5 with the two-barrier sweeps); larger ones,
+// which come first, by a CTA each that runs the whole windowed iteration
+// (batch_big.cuh), as a sweep that touches global memory at every step costs
+// several times the windows and their updates.  With 128 threads (an
+// autotuned or chosen configuration) one launch solves all by small-bulge
+// multishift sweeps (cta_small_qz_ms), in place in global memory above
+// smem_max.  beta >= 0, eigenvalues and per-pencil status words at the end;
+// no host round trip.
 #include <cuda_runtime.h>
 #include <float.h>
 #include <stdint.h>
@@ -21,6 +25,7 @@
 #include <mutex>
 
 #include "../../include/b200qz.h"
+#include "batch_big.cuh"
 #include "kernels.h"
 #include "qz_roles.cuh"
 
@@ -159,36 +164,99 @@ __global__ void __launch_bounds__(kBatchThreads, 1) k_batch_qz(int count, const 
   }
 }
 
+// Pencils above kBatchSmemMax, one CTA each from the same kind of queue.
+__global__ void __launch_bounds__(kBigThreads, 1) k_batch_big(int count, const int* __restrict__ order,
+                                                              const int* __restrict__ nsz,
+                                                              const int64_t* __restrict__ moff,
+                                                              const int64_t* __restrict__ eoff, double* H, double* T,
+                                                              double* Q, double* Z, double* AR, double* AI,
+                                                              double* BE, int* status, int* counter) {
+  extern __shared__ double smem[];
+  __shared__ int s_next;
+  __shared__ double red[32];
+  __shared__ int si[64];
+  for (;;) {
+    if (threadIdx.x == 0) s_next = atomicAdd(counter, 1);
+    __syncthreads();
+    const int idx = s_next;
+    __syncthreads();
+    if (idx >= count) break;
+    const int q = order[idx];
+    BigPencil p{H + moff[q], T + moff[q], Q + moff[q], Z + moff[q], nsz[q], {}};
+    const int n = p.n;
+    double hs = 0.0, ts = 0.0;
+    for (int j = threadIdx.x >> 5; j < n; j += kBigThreads / 32)
+      for (int i = threadIdx.x & 31; i < n; i += 32) {
+        const size_t k = i + (size_t)j * n;
+        hs += p.H[k] * p.H[k];
+        ts += p.T[k] * p.T[k];
+        p.Q[k] = p.Z[k] = i == j ? 1.0 : 0.0;
+      }
+    hs = block_sum(hs, red);
+    ts = block_sum(ts, red);
+    p.tol.safmin = DBL_MIN;
+    p.tol.ulp = DBL_EPSILON;
+    p.tol.smlnum = DBL_MIN * ((double)n / DBL_EPSILON);
+    p.tol.htol = fmax(DBL_MIN, DBL_EPSILON * sqrt(hs));
+    p.tol.ttol = fmax(DBL_MIN, DBL_EPSILON * sqrt(ts));
+    const int info = big_solve(p, smem, 30 * n);
+    __syncthreads();
+    if (info == 0) {
+      BigExecAll x{(int)threadIdx.x, kBigThreads, si, smem};
+      WinState w;
+      w.n = n;
+      w.H = MatV{p.H, n}; w.T = MatV{p.T, n}; w.Q = MatV{p.Q, n}; w.Z = MatV{p.Z, n};
+      w.wantq = w.wantz = true;
+      w.tol = p.tol;
+      cta_finalize(x, w, AR + eoff[q], AI + eoff[q], BE + eoff[q]);
+    }
+    if (threadIdx.x == 0) status[q] = info;
+    __syncthreads();
+  }
+}
+
 // H, T, Q, Z, then the role buffer and the standardisation's 3n doubles
 size_t batch_smem_bytes(int smem_max) {
   return ((size_t)4 * smem_max * smem_ld(smem_max) + kRoleDoubles + 3 * (size_t)smem_max) * sizeof(double);
 }
 
 cudaError_t batch_init() {
+  const cudaError_t e = cudaFuncSetAttribute(k_batch_big, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBigSmem);
+  if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(k_batch_qz, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)batch_smem_bytes(kBatchSmemMax));
 }
 
-void launch_batch(cudaStream_t st, int grid, int threads, int smem_max, int count, const int* order, const int* nsz,
-                  const int64_t* moff, const int64_t* eoff, double* H, double* T, double* Q, double* Z, double* AR,
-                  double* AI, double* BE, int* status, int* counter) {
-  cudaMemsetAsync(counter, 0, sizeof(int), st);
-  k_batch_qz<<<grid, threads, batch_smem_bytes(smem_max), st>>>(count, order, nsz, moff, eoff, H, T, Q, Z, AR, AI, BE,
-                                                                status, counter, smem_max);
-}
-
-// The same launch, returning the status of this call's own memset and
-// kernel launch (cudaLaunchKernel reports the launch error directly, so an
-// error left pending by unrelated earlier work is neither reported as ours
-// nor cleared).
-static cudaError_t launch_batch_checked(cudaStream_t st, int grid, int threads, int smem_max, int count,
-                                        const int* order, const int* nsz, const int64_t* moff, const int64_t* eoff,
-                                        double* H, double* T, double* Q, double* Z, double* AR, double* AI,
-                                        double* BE, int* status, int* counter) {
-  cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(int), st);
+// Two launches: the pencils above kBatchSmemMax (the first nbig of the order;
+// none with 128 threads, which keep the one-kernel form), then the others.
+// Returns the status of this call's own memset and launches (cudaLaunchKernel
+// reports the launch error directly, so an error left pending by unrelated
+// earlier work is neither reported as ours nor cleared).
+cudaError_t launch_batch(cudaStream_t st, int grid, int threads, int smem_max, int count, int nbig, int sm_count,
+                         const int* order, const int* nsz, const int64_t* moff, const int64_t* eoff, double* H,
+                         double* T, double* Q, double* Z, double* AR, double* AI, double* BE, int* status,
+                         int* counter) {
+  cudaError_t e = cudaMemsetAsync(counter, 0, 2 * sizeof(int), st);
   if (e != cudaSuccess) return e;
+  if (threads != kRoleThreads) nbig = 0;
+  if (nbig > 0) {
+    void* args[] = {&nbig, &order, &nsz, &moff, &eoff, &H, &T, &Q, &Z, &AR, &AI, &BE, &status, &counter};
+    e = cudaLaunchKernel((const void*)k_batch_big, dim3(std::min(nbig, sm_count)), dim3(kBigThreads), args, kBigSmem,
+                         st);
+    if (e != cudaSuccess) return e;
+  }
+  count -= nbig;
+  order += nbig;
+  counter += 1;
+  if (count == 0) return cudaSuccess;
   void* args[] = {&count, &order, &nsz, &moff, &eoff, &H, &T, &Q, &Z, &AR, &AI, &BE, &status, &counter, &smem_max};
   return cudaLaunchKernel((const void*)k_batch_qz, dim3(grid), dim3(threads), args, batch_smem_bytes(smem_max), st);
+}
+
+int batch_big_count(const int* n, int count) {
+  int k = 0;
+  for (int i = 0; i < count; ++i) k += n[i] > kBatchSmemMax;
+  return k;
 }
 
 // ---------------------------------------------------------------------------
@@ -205,7 +273,7 @@ static cudaError_t launch_batch_checked(cudaStream_t st, int grid, int threads, 
 namespace {
 
 constexpr int kNoAllocMaxPencils = 4096;
-// moff, eoff (int64), order, n (int32), queue counter
+// moff, eoff (int64), order, n (int32), two queue counters
 constexpr size_t kNoAllocBytes = (size_t)kNoAllocMaxPencils * (2 * sizeof(int64_t) + 2 * sizeof(int)) + 256;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
@@ -276,9 +344,10 @@ extern "C" int b200qz_solve_batched_noalloc(int count, const int* n, const long 
       cudaMemcpyAsync(d_order, order, count * sizeof(int), cudaMemcpyHostToDevice, st) != cudaSuccess ||
       cudaMemcpyAsync(d_n, n, count * sizeof(int), cudaMemcpyHostToDevice, st) != cudaSuccess)
     return 10001;
-  // the queue counter is zeroed on the stream before the kernel starts
-  const cudaError_t e = launch_batch_checked(st, d->sm_count, kRoleThreads, kBatchSmemMax, count, d_order, d_n, d_moff, d_eoff,
-                                             h, t, q, z, alphar, alphai, beta, info, d_counter);
+  // the queue counters are zeroed on the stream before the kernels start
+  const cudaError_t e =
+      launch_batch(st, d->sm_count, kRoleThreads, kBatchSmemMax, count, batch_big_count(n, count), d->sm_count,
+                   d_order, d_n, d_moff, d_eoff, h, t, q, z, alphar, alphai, beta, info, d_counter);
   return e == cudaSuccess ? 0 : 10001;
 }
 

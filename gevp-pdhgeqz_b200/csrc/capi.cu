@@ -82,11 +82,12 @@ struct BatchKey {
   // descriptors (order, n, queue counter, moff, eoff), then h, t, q, z,
   // alphar, alphai, beta, info
   const void* ptr[13] = {};
-  int count = -1, threads = 0, smem_max = 0, ctas_per_sm = 0;
+  int count = -1, threads = 0, smem_max = 0, ctas_per_sm = 0, nbig = 0;
   bool operator==(const BatchKey& o) const {
     for (int i = 0; i < 13; ++i)
       if (ptr[i] != o.ptr[i]) return false;
-    return count == o.count && threads == o.threads && smem_max == o.smem_max && ctas_per_sm == o.ctas_per_sm;
+    return count == o.count && threads == o.threads && smem_max == o.smem_max && ctas_per_sm == o.ctas_per_sm &&
+           nbig == o.nbig;
   }
 };
 
@@ -642,7 +643,7 @@ int b200qz_set_params(b200qz_ctx* c, int nw_max, int w_chase, int nmin, int nibb
   if (nibble >= 0) c->params.nibble = nibble;
   if (ns_max >= 0) c->params.ns_max = ns_max;
   if (maxit_factor >= 0) c->params.maxit_factor = std::max(1, maxit_factor);
-  c->params.chain_max = std::min(kMaxChain, std::max(1, (c->params.w_chase - 4) / 6));
+  if (w_chase >= 0) c->params.chain_max = std::min(kMaxChain, std::max(1, (c->params.w_chase - 4) / 6));
   return 0;
 }
 
@@ -918,8 +919,8 @@ extern "C" int b200qz_solve_batched_dev(b200qz_ctx* c, int count, const int* n, 
   int *d_order, *d_n, *d_counter;
   int64_t *d_moff, *d_eoff;
   if (batch_prepare(c, count, n, moff, eoff, &d_order, &d_n, &d_counter, &d_moff, &d_eoff) != 0) return 10001;
-  // one persistent launch, captured in a CUDA graph and replayed while
-  // every operand pointer, the count and the configuration stay the same
+  // the persistent launches, captured in a CUDA graph and replayed while
+  // every operand pointer, the counts and the configuration stay the same
   BatchKey key;
   const void* ops[13] = {d_order, d_n, d_counter, d_moff, d_eoff, h, t, q, z, alphar, alphai, beta, info};
   for (int i = 0; i < 13; ++i) key.ptr[i] = ops[i];
@@ -927,12 +928,13 @@ extern "C" int b200qz_solve_batched_dev(b200qz_ctx* c, int count, const int* n, 
   key.threads = c->batch_threads;
   key.smem_max = c->batch_smem_max;
   key.ctas_per_sm = c->batch_ctas_per_sm;
+  key.nbig = batch_big_count(n, count);
   if (!c->bexec || !(key == c->bkey)) {
     if (c->bexec) { cudaGraphExecDestroy(c->bexec); c->bexec = nullptr; }
     if (c->bgraph) { cudaGraphDestroy(c->bgraph); c->bgraph = nullptr; }
     QZ_CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    launch_batch(c->stream, batch_grid(c), c->batch_threads, c->batch_smem_max, count, d_order, d_n, d_moff, d_eoff,
-                 h, t, q, z, alphar, alphai, beta, info, d_counter);
+    QZ_CK(launch_batch(c->stream, batch_grid(c), c->batch_threads, c->batch_smem_max, count, key.nbig, c->sm_count,
+                       d_order, d_n, d_moff, d_eoff, h, t, q, z, alphar, alphai, beta, info, d_counter));
     QZ_CK(cudaStreamEndCapture(c->stream, &c->bgraph));
     if (c->err == cudaSuccess) QZ_CK(cudaGraphInstantiate(&c->bexec, c->bgraph, 0));
     if (c->err != cudaSuccess) return 10001;

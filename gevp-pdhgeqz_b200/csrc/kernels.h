@@ -22,9 +22,12 @@ constexpr int kBatchThreads = 256;
 constexpr int kBatchSmemMax = 80;
 size_t batch_smem_bytes(int smem_max);
 cudaError_t batch_init();
-void launch_batch(cudaStream_t st, int grid, int threads, int smem_max, int count, const int* order, const int* nsz,
-                  const int64_t* moff, const int64_t* eoff, double* H, double* T, double* Q, double* Z, double* AR,
-                  double* AI, double* BE, int* status, int* counter);
+cudaError_t launch_batch(cudaStream_t st, int grid, int threads, int smem_max, int count, int nbig, int sm_count,
+                         const int* order, const int* nsz, const int64_t* moff, const int64_t* eoff, double* H,
+                         double* T, double* Q, double* Z, double* AR, double* AI, double* BE, int* status,
+                         int* counter);
+// pencils above kBatchSmemMax
+int batch_big_count(const int* n, int count);
 
 // chains chased concurrently (one CTA each) by one wave launch
 constexpr int kMaxWave = 8;

@@ -42,12 +42,17 @@ constexpr int kUpdThreads = 128;   // 4 warps (per-tile kernels)
 constexpr int kUpdMaxThreads = 512;  // persistent kernels: two warps per 16-row slice, up to 16
 constexpr int kUpdMaxK = 128;      // fast path limit
 
-#ifdef QZ_DEFINE_UPDATE_KERNELS
+constexpr int kUpdRightLd = kUpdTile + 4;  // right slab tile in shared memory
+
+#ifdef __CUDACC__
 __device__ __forceinline__ void dmma_8x8x4(double& d0, double& d1, double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
                : "+d"(d0), "+d"(d1)
                : "d"(a), "d"(b));
 }
+#endif
+
+#ifdef QZ_DEFINE_UPDATE_KERNELS
 
 __device__ __forceinline__ int upd_find_job(const UpdBatch& B, int& tile) {
   int t = blockIdx.x;
@@ -265,8 +270,6 @@ __device__ __forceinline__ void upd_stage(const UpdJob& J, int tile, int side, d
     upd_copy(Xs, ldx, J.M + r0 + (int64_t)J.c0 * J.ld, J.ld, min(kUpdTile, J.r0 + J.len - r0), J.k, kUpdTile, kp);
   }
 }
-
-constexpr int kUpdRightLd = kUpdTile + 4;
 
 template <int SIDE>
 __global__ void __launch_bounds__(kUpdMaxThreads) k_update_persist(UpdBatch B, int total) {
