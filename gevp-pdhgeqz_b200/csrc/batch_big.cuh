@@ -5,9 +5,11 @@
 //
 // Windows live in shared memory; a window's factors update the rest of H and
 // T, Q and Z in 32-wide slab tiles on the FP64 tensor cores (two groups of
-// eight warps, a tile each).  Bound: per chase window of 64 rows the chase
-// steps (about 45 us) and the updates (4 n / 32 tiles at one SM's FP64 rate,
-// about 50 us at n = 300).
+// eight warps, a tile each).  What bounds it, at n = 300 with every SM
+// occupied (about 80 ms a pencil): the early deflations, 45 % (52 of 1.3M
+// cycles: serial chains of rotations), the updates, 30 % (300 of 160k
+// cycles, 2.4 times the tensor rate, as 148 pencils' matrices do not stay in
+// L2), and the chases, 22 % (115k cycles each: a serial chain of reflectors).
 #pragma once
 #include "qz_chase_roles.cuh"
 #include "update.cuh"
@@ -110,93 +112,135 @@ __device__ inline void big_store(const BigPencil& p, int w, int wk, const double
   __syncthreads();
 }
 
-// M(w:w+k, c:c+cols) <- W^T M (left) or M(r:r+rows, w:w+k) <- M W (right) for
-// one 32-wide tile, by the 256 threads of group grp; W in shared memory.
-__device__ inline void big_tile(bool left, double* M, int n, int w, int k, int o, int len, const double* W, int ldw,
-                                double* X, int grp) {
-  const int tid = threadIdx.x & 255, warp = tid >> 5, lane = tid & 31, lr = lane >> 2, lc = lane & 3;
-  const int kp = (k + 15) & ~15, lim = len < kUpdTile ? len : kUpdTile;
-  const int ldx = left ? kBigEnd + 4 : kUpdRightLd;
-  auto bar = [&]() { asm volatile("bar.sync %0, 256;" ::"r"(3 + grp) : "memory"); };
-  if (left) {
-    for (int j = warp; j < kUpdTile; j += 8)
-      for (int i = lane; i < kp; i += 32)
-        X[i + j * ldx] = (i < k && j < lim) ? M[(size_t)(w + i) + (size_t)(o + j) * n] : 0.0;
-  } else {
-    for (int j = warp; j < kp; j += 8)
-      X[lane + j * ldx] = (lane < lim && j < k) ? M[(size_t)(o + lane) + (size_t)(w + j) * n] : 0.0;
-  }
-  bar();
-  const int half = warp & 1;
-  for (int sl = warp >> 1; sl < kp / 16; sl += 4) {
-    double acc[2][2][2] = {};
-    for (int kk = 0; kk < kp; kk += 4) {
-      double wf[2], xf[2];
+// A tile of an update: M(w:w+k, o:o+len) <- W^T M (left) or M(o:o+len, w:w+k)
+// <- M W (right), at most 32 of the other dimension.
+struct BigTile {
+  double* M;
+  const double* W;
+  int o, len;
+};
+constexpr int kBigSlabLd = kBigEnd + 4;                 // left slab tile
+constexpr int kBigSlab = kBigEnd * kUpdRightLd;         // doubles of a group's tile
+constexpr int kBigHold = 3 * (kUpdTile / 8);            // elements of a tile per thread
+static_assert(kBigSlabLd * kUpdTile <= kBigSlab, "slab tile");
+static_assert(kBigEnd <= 96 && kBigEnd <= 8 * kBigHold, "elements held");
+
+// The thread's elements of a tile, zero outside it.  Left: rows lane,
+// lane + 32, lane + 64 of columns warp, warp + 8, ..; right: row lane of
+// columns warp, warp + 8, ..
+template <bool kLeft>
+__device__ __forceinline__ void big_fetch(const BigTile& t, int n, int w, int k, double (&v)[kBigHold]) {
+  const int warp = (threadIdx.x & 255) >> 5, lane = threadIdx.x & 31;
 #pragma unroll
-      for (int a = 0; a < 2; ++a) {
-        const int i = kk + lc, j = sl * 16 + a * 8 + lr;
-        wf[a] = (i < k && j < k) ? W[i + j * ldw] : 0.0;
-        xf[a] = left ? X[i + (half * 16 + a * 8 + lr) * ldx] : X[half * 16 + a * 8 + lr + i * ldx];
+  for (int e = 0; e < kBigHold; ++e) {
+    const int i = kLeft ? lane + 32 * (e % 3) : lane, j = warp + 8 * (kLeft ? e / 3 : e);
+    const bool in = kLeft ? (i < k && j < t.len) : (i < t.len && j < k);
+    v[e] = in ? t.M[kLeft ? (size_t)(w + i) + (size_t)(t.o + j) * n : (size_t)(t.o + i) + (size_t)(w + j) * n] : 0.0;
+  }
+}
+template <bool kLeft>
+__device__ __forceinline__ void big_put(double* X, int kp, const double (&v)[kBigHold]) {
+  const int warp = (threadIdx.x & 255) >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int e = 0; e < kBigHold; ++e) {
+    const int i = kLeft ? lane + 32 * (e % 3) : lane, j = warp + 8 * (kLeft ? e / 3 : e);
+    if (kLeft ? i < kp : j < kp) X[kLeft ? i + j * kBigSlabLd : i + j * kUpdRightLd] = v[e];
+  }
+}
+
+// The tiles t = grp, grp + 2, .. below count, by the 256 threads of group
+// grp; W in shared memory.  The next tile's elements are read while this
+// one's product runs: with the reads waited for, the updates of a window of
+// 64 rows at n = 320 took 199k cycles, with them ahead 156k (24 tiles, 2.0k
+// cycles each at the SM's FP64 tensor rate, on two groups).
+template <bool kLeft, class TileOf>
+__device__ __forceinline__ void big_tiles(const TileOf& tile_of, int count, int n, int w, int k, int ldw, double* X,
+                                          int grp) {
+  const int warp = (threadIdx.x & 255) >> 5, lane = threadIdx.x & 31, lr = lane >> 2, lc = lane & 3;
+  const int kp = (k + 15) & ~15, half = warp & 1;
+  auto bar = [&]() { asm volatile("bar.sync %0, 256;" ::"r"(3 + grp) : "memory"); };
+  double v[kBigHold];
+  BigTile t{};
+  if (grp < count) {
+    t = tile_of(grp);
+    big_fetch<kLeft>(t, n, w, k, v);
+  }
+  for (int q = grp; q < count; q += 2) {
+    bar();  // the last product has read the slab
+    big_put<kLeft>(X, kp, v);
+    bar();
+    const BigTile now = t;
+    if (q + 2 < count) {
+      t = tile_of(q + 2);
+      big_fetch<kLeft>(t, n, w, k, v);
+    }
+    for (int sl = warp >> 1; sl < kp / 16; sl += 4) {
+      double acc[2][2][2] = {};
+      for (int kk = 0; kk < kp; kk += 4) {
+        double wf[2], xf[2];
+#pragma unroll
+        for (int a = 0; a < 2; ++a) {
+          const int i = kk + lc, j = sl * 16 + a * 8 + lr;
+          wf[a] = (i < k && j < k) ? now.W[i + j * ldw] : 0.0;
+          xf[a] = kLeft ? X[i + (half * 16 + a * 8 + lr) * kBigSlabLd] : X[half * 16 + a * 8 + lr + i * kUpdRightLd];
+        }
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+          for (int b = 0; b < 2; ++b)
+            dmma_8x8x4(acc[a][b][0], acc[a][b][1], kLeft ? wf[a] : xf[a], kLeft ? xf[b] : wf[b]);
       }
 #pragma unroll
       for (int a = 0; a < 2; ++a)
 #pragma unroll
         for (int b = 0; b < 2; ++b)
-          dmma_8x8x4(acc[a][b][0], acc[a][b][1], left ? wf[a] : xf[a], left ? xf[b] : wf[b]);
-    }
 #pragma unroll
-    for (int a = 0; a < 2; ++a)
-#pragma unroll
-      for (int b = 0; b < 2; ++b)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int x = a * 8 + lr, y = b * 8 + lc * 2 + e;
-          if (left) {
-            const int i = sl * 16 + x, j = half * 16 + y;
-            if (i < k && j < lim) M[(size_t)(w + i) + (size_t)(o + j) * n] = acc[a][b][e];
-          } else {
-            const int i = half * 16 + x, j = sl * 16 + y;
-            if (i < lim && j < k) M[(size_t)(o + i) + (size_t)(w + j) * n] = acc[a][b][e];
+          for (int e = 0; e < 2; ++e) {
+            const int x = a * 8 + lr, y = b * 8 + lc * 2 + e;
+            const int i = kLeft ? sl * 16 + x : half * 16 + x, j = kLeft ? half * 16 + y : sl * 16 + y;
+            if (kLeft ? (i < k && j < now.len) : (i < now.len && j < k))
+              now.M[kLeft ? (size_t)(w + i) + (size_t)(now.o + j) * n : (size_t)(now.o + i) + (size_t)(w + j) * n] =
+                  acc[a][b][e];
           }
-        }
+    }
   }
-  bar();
 }
 
 // The window's factors on the rest: H, T right of it, then H, T above it and
-// Q, Z.  X: two slab buffers.
+// Q, Z.  X: two slab tiles.
 __device__ inline void big_update(const BigPencil& p, int w, int wk, const double* U, const double* V, int ldu,
                                   double* X) {
   const int grp = threadIdx.x >> 8, n = p.n;
-  double* const Xg = X + grp * (kBigEnd + 16) * (kUpdTile + 4);
+  double* const Xg = X + grp * kBigSlab;
   const int right = n - (w + wk), tr = (right + kUpdTile - 1) / kUpdTile;
-  for (int t = grp; t < 2 * tr; t += 2) {
-    double* const M = t < tr ? p.H : p.T;
-    const int c = (t < tr ? t : t - tr) * kUpdTile;
-    big_tile(true, M, n, w, wk, w + wk + c, right - c, U, ldu, Xg, grp);
-  }
+  big_tiles<true>(
+      [&](int t) {
+        const int c = (t < tr ? t : t - tr) * kUpdTile;
+        return BigTile{t < tr ? p.H : p.T, U, w + wk + c, right - c};
+      },
+      2 * tr, n, w, wk, ldu, Xg, grp);
   __syncthreads();
   const int ta = (w + kUpdTile - 1) / kUpdTile, tq = (n + kUpdTile - 1) / kUpdTile;
-  for (int t = grp; t < 2 * ta + 2 * tq; t += 2) {
-    if (t < 2 * ta) {
-      const int r = (t < ta ? t : t - ta) * kUpdTile;
-      big_tile(false, t < ta ? p.H : p.T, n, w, wk, r, w - r, V, ldu, Xg, grp);
-    } else {
-      const int u = t - 2 * ta, r = (u < tq ? u : u - tq) * kUpdTile;
-      big_tile(false, u < tq ? p.Q : p.Z, n, w, wk, r, n - r, u < tq ? U : V, ldu, Xg, grp);
-    }
-  }
+  big_tiles<false>(
+      [&](int t) {
+        if (t < 2 * ta) {
+          const int r = (t < ta ? t : t - ta) * kUpdTile;
+          return BigTile{t < ta ? p.H : p.T, V, r, w - r};
+        }
+        const int u = t - 2 * ta, r = (u < tq ? u : u - tq) * kUpdTile;
+        return BigTile{u < tq ? p.Q : p.Z, u < tq ? U : V, r, n - r};
+      },
+      2 * ta + 2 * tq, n, w, wk, ldu, Xg, grp);
   __syncthreads();
 }
-// slab buffers: behind the four windows of order wk (the larger windows use
-// the H and T windows, which are stored by then)
-__device__ inline double* big_slab(const BigMem& m, int wk) {
-  const int ld = big_ld(wk);
-  const int used = 4 * wk * ld;
-  constexpr int need = 2 * (kBigEnd + 16) * (kUpdTile + 4);
-  return used + need <= 4 * kBigWin ? m.win + used : m.win;
+// slab tiles: behind the used part of the windows, or in the H and T windows
+// (stored by then) of the larger ones
+__device__ inline double* big_slab(const BigMem& m, int used) {
+  return used + 2 * kBigSlab <= 4 * kBigWin ? m.win + used : m.win;
 }
-static_assert(2 * (kBigEnd + 16) * (kUpdTile + 4) <= 2 * kBigWin, "slab buffers in the H and T windows");
+// with U at 2 wk ld: the largest window whose slab tiles do not fit behind is
+// at least this wide, and H and T hold them
+static_assert(4 * 70 * 71 + 2 * kBigSlab <= 4 * kBigWin && 2 * kBigSlab <= 2 * 70 * 71, "slab tiles");
 
 // deflation scan: ktop, zeros on T's diagonal (k_scan)
 __device__ inline void big_scan(const BigPencil& p, int ifirst, int kbot, BigShare* sh) {
@@ -257,6 +301,44 @@ __device__ inline int big_pairs(const double* sr, const double* si, const double
   return np;
 }
 
+// The window phases are functions of their own, which take the shared memory
+// by itself (not through pointers, whose accesses would be generic): inlined,
+// the solve's state on top of theirs made it spill more of the 128 registers
+// that 512 threads leave (220 pencils of order 32 to 300: 106 ms, 96 so).
+
+// window QZ and early deflation of the loaded window of order n (k_aed_win),
+// by the first kRoleThreads threads
+static __device__ __noinline__ void big_aed(int n, Tol tol, double s, int nskip) {
+  extern __shared__ double smem[];
+  const BigMem m = big_mem(smem);
+  const int ld = big_ld(n);
+  BigExec x{(int)threadIdx.x, kRoleThreads, m.sh->si, m.sd};
+  RoleBuf* const rb = (RoleBuf*)m.ring;
+  WinState w;
+  w.n = n;
+  w.H = MatV{m.win, ld};
+  w.T = MatV{m.win + n * ld, ld};
+  w.Q = MatV{m.win + 2 * n * ld, ld};
+  w.Z = MatV{m.win + 3 * n * ld, ld};
+  w.wantq = w.wantz = true;
+  w.tol = tol;
+  const int qz = cta_role_qz(x, w, 30 * n, rb);
+  if (qz == 0) cta_std_all(x, w, m.sd + 64);
+  double* const sr = m.sh->shift;
+  cta_aed_deflate(
+      x, w, s, sr, sr + kBigShifts, sr + 2 * kBigShifts, qz,
+      [&]() { return cta_role_spike(x, w, s, nskip, false, rb); },
+      [&](int mm) { return cta_role_hessred(x, w, mm, rb); });
+}
+
+// chase of the loaded window of order wk (k_chase_win)
+static __device__ __noinline__ bool big_chase(int wk, int last, int ld, int ldu, int nb, int tmax) {
+  extern __shared__ double smem[];
+  const BigMem m = big_mem(smem);
+  return cta_chase_roles(wk, last, MatV{m.win, ld}, MatV{m.win + wk * ld, ld}, MatV{m.win + 2 * wk * ld, ldu},
+                         MatV{m.win + wk * (2 * ld + ldu), ldu}, m.sh->bl, nb, tmax, m.ring, &m.sh->chase);
+}
+
 // The whole solve; 0, or the 1-based row where it stopped.
 __device__ inline int big_solve(const BigPencil& p, double* smem, int maxit) {
   const BigMem m = big_mem(smem);
@@ -300,7 +382,7 @@ __device__ inline int big_solve(const BigPencil& p, double* smem, int maxit) {
         cta_inf_window(x, wk, ktop >= w ? ktop - w : -1, jz - w, stop - w, stop == kbot, MatV{Hs, ld}, MatV{Ts, ld},
                        MatV{Us, ld}, MatV{Vs, ld});
         big_store(p, w, wk, Hs, Ts, ld);
-        big_update(p, w, wk, Us, Vs, ld, big_slab(m, wk));
+        big_update(p, w, wk, Us, Vs, ld, big_slab(m, 4 * wk * ld));
         if (stop == kbot) break;
         jz = stop;
       }
@@ -316,28 +398,13 @@ __device__ inline int big_solve(const BigPencil& p, double* smem, int maxit) {
       double *Hs = m.win, *Ts = Hs + nw * ld, *Us = Ts + nw * ld, *Vs = Us + nw * ld;
       big_load(p, kwtop, nw, Hs, Ts, Us, Vs, ld, ld);
       const double s = whole ? 0.0 : p.H[kwtop + (size_t)(kwtop - 1) * n];
-      if (tid < kRoleThreads) {
-        BigExec x{tid, kRoleThreads, sh->si, m.sd};
-        RoleBuf* const rb = (RoleBuf*)m.ring;
-        WinState ws;
-        ws.n = nw;
-        ws.H = MatV{Hs, ld}; ws.T = MatV{Ts, ld}; ws.Q = MatV{Us, ld}; ws.Z = MatV{Vs, ld};
-        ws.wantq = ws.wantz = true;
-        ws.tol = p.tol;
-        const int qz = cta_role_qz(x, ws, 30 * nw, rb);
-        if (qz == 0) cta_std_all(x, ws, m.sd + 64);
-        double* const sr = sh->shift;
-        cta_aed_deflate(
-            x, ws, s, sr, sr + kBigShifts, sr + 2 * kBigShifts, qz,
-            [&]() { return cta_role_spike(x, ws, s, whole ? 0 : 4, false, rb); },
-            [&](int mm) { return cta_role_hessred(x, ws, mm, rb); });
-      }
+      if (tid < kRoleThreads) big_aed(nw, p.tol, s, whole ? 0 : 4);
       __syncthreads();
       const int mu = sh->si[8], status = sh->si[9], changed = sh->si[10];
       if (status == 0 && changed) {
         if (!whole && tid == 0) p.H[kwtop + (size_t)(kwtop - 1) * n] = s * Us[0];
         big_store(p, kwtop, nw, Hs, Ts, ld);
-        big_update(p, kwtop, nw, Us, Vs, ld, big_slab(m, nw));
+        big_update(p, kwtop, nw, Us, Vs, ld, big_slab(m, 4 * nw * ld));
       }
       if (whole) {
         if (status != 0) return kbot + 1;
@@ -394,14 +461,14 @@ __device__ inline int big_solve(const BigPencil& p, double* smem, int maxit) {
                               sh->poly[3 * (p0 + k) + 1], sh->poly[3 * (p0 + k) + 2]};
           if (k == nb - 1) top = w + base + thi;
         }
-        const int ld = big_ld(wk);
-        double *Hs = m.win, *Ts = Hs + wk * ld, *Us = Ts + wk * ld, *Vs = Us + wk * ld;
-        big_load(p, w, wk, Hs, Ts, Us, Vs, ld, ld);
-        const bool ok = cta_chase_roles(wk, last, MatV{Hs, ld}, MatV{Ts, ld}, MatV{Us, ld}, MatV{Vs, ld}, sh->bl, nb,
-                                        tmax, m.ring, &sh->chase);
+        // U, V: fragments of the updates on distinct banks
+        const int ld = big_ld(wk), ldu = ((wk + 7) & ~7) + 4;
+        double *Hs = m.win, *Ts = Hs + wk * ld, *Us = Ts + wk * ld, *Vs = Us + wk * ldu;
+        big_load(p, w, wk, Hs, Ts, Us, Vs, ld, ldu);
+        const bool ok = big_chase(wk, last, ld, ldu, nb, tmax);
         if (!ok) return kbot + 1;
         big_store(p, w, wk, Hs, Ts, ld);
-        big_update(p, w, wk, Us, Vs, ld, big_slab(m, wk));
+        big_update(p, w, wk, Us, Vs, ldu, big_slab(m, 2 * wk * (ld + ldu)));
         if (fin) break;
         first = false;
       }

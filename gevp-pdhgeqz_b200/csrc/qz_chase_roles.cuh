@@ -343,7 +343,7 @@ __device__ inline bool cta_chase_roles(int wk, int last, MatV H, MatV T, MatV U,
       if (sh->stop != 0) break;
     }
   } else {
-    const int warp = wid >> 2, f = 32 * warp + lane;
+    const int warp = wid >> 2, f = 32 * warp + lane, ldf = U.ld;
     for (int tau = 0; tau < tmax; ++tau) {
       bool ok = false;
       for (int it = 0; it < kRoleSpin; ++it) {
@@ -370,14 +370,14 @@ __device__ inline bool cta_chase_roles(int wk, int last, MatV H, MatV T, MatV U,
             kj[i] = *(const int2*)(r + 8);
             if (b0 + i >= nb) kj[i].x = 0;
             h[i] = chase_rec(r, off);
-            const double* q = row + (kj[i].x == 1 ? kj[i].y : 0) * ld;
-            x0[i] = q[0]; x1[i] = q[ld]; x2[i] = q[2 * ld];
+            const double* q = row + (kj[i].x == 1 ? kj[i].y : 0) * ldf;
+            x0[i] = q[0]; x1[i] = q[ldf]; x2[i] = q[2 * ldf];
           }
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             house3_apply(h[i], x0[i], x1[i], x2[i]);
-            role_put3(kj[i].x == 1, role_sm(row + kj[i].y * ld), 8 * ld, x0[i], x1[i], x2[i]);
-            if (kj[i].x == 2) rot_vec(h[i].s, h[i].u0, row + kj[i].y * ld, ld);
+            role_put3(kj[i].x == 1, role_sm(row + kj[i].y * ldf), 8 * ldf, x0[i], x1[i], x2[i]);
+            if (kj[i].x == 2) rot_vec(h[i].s, h[i].u0, row + kj[i].y * ldf, ldf);
           }
         }
       }
