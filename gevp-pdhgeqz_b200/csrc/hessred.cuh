@@ -10,17 +10,15 @@
 // (lartg(B(J, J), B(J, J-1))).  G acts on A(.., jc+1:n) and B(.., J-1:n),
 // Z on A(0:ihi, ..) and B(0:J-1, ..); Q accumulates G and Z accumulates Z.
 //
-// Device form.  The pairs of one column form a dependent chain through the
+// Windowed form.  The pairs of one column form a dependent chain through the
 // 2x2 diagonal blocks of B; everything else is a rotation applied to a row
 // or a column "walk".  A column's chain runs in windows of at most W pairs
-// from the bottom up.  One CTA holds the window's diagonal block of B in
-// shared memory with the column's entries of A: one thread computes the
-// row rotations from the column of A (hr_g_chain, which does not depend on
-// B) ahead of the others, which run the column rotations through the block
-// (cta_hr_zchain: one barrier per pair, the block thread one pair ahead of
-// the threads applying the previous pair inside the block).  The rest of a
-// window's rotations is applied by the launch of the next window (or by the
-// column's last launch) as walks:
+// from the bottom up, on the window's diagonal block of B and the column's
+// entries of A; the row rotations come from the column of A alone.  The rest
+// of a window's rotations is applied with the next window (or after the
+// column's last) as walks.  This file has the pieces one thread can run
+// (hr_g_chain, cta_hr_zchain and the walks, by which the form is checked on
+// the host); hessred.cu has the device's split of them.  The walks:
 //   (a) its Z on the rows of B the next window's block holds (CTA 0),
 //   (e) its Z on the rows of B above those,
 //   (f) its G on the columns of B right of the window,
@@ -200,7 +198,7 @@ QZ_HD void hr_g_chain(int m, double* acol, double* gbuf, int* gready) {
   for (int J = 1; J < m; ++J) acol[J] = 0.0;
 }
 
-// The column rotations of one window (the chain threads): pairs J = m-1
+// The column rotations of one window (threads of an executor, or one): pairs J = m-1
 // .. 1 on the diagonal block Tw (m x m, ld ldw, upper triangular), pair
 // J's row rotation read from gbuf once *gready >= m-J (x.wait).  On return
 // Tw is the block after the window's rotations and gbuf[4J+2..4J+3] holds
