@@ -11,10 +11,10 @@
 // forms 32 at a time from a scan of squares.  G on the block's own columns is
 // left to the walks (f) (Z's of later windows do not reach those entries).
 // The other CTAs apply the previous window's rotations elsewhere (walks (e),
-// (f), (g)) on entries CTA 0 does not touch; in a column's first launch, which
-// has no previous window, they apply the previous column's factors to Q and
-// Z (two sets of rotation records).  After the column's last window, one
-// launch applies that window's walks and one the column's G to A.
+// (f), (g)) on entries CTA 0 does not touch, and the pairs of the window's
+// rows of the previous column's factors to Q and Z (two sets of rotation
+// records).  After the column's last window, one launch applies that window's
+// walks and one the column's G to A.
 //
 // Walks along rows (a lane per row, loads of 32 rows coalesced, 16 ahead of
 // the carry) take the Z's and Q; walks down columns (a warp per column, 32
@@ -25,7 +25,7 @@
 // issue of a lone warp), 760 with a barrier per pair; then a window's loads
 // and stores through that SM, 16 bytes a cycle.  All in, n = 800 with Q and
 // Z: 272 ms then, 86 now (windows of 64 to 160 pairs within 7 % of that);
-// n = 2000: 1.79 s then, 0.57 now.
+// n = 2000: 1.79 s then, 0.53 now.
 #include "hessred.h"
 
 #include <algorithm>
@@ -202,18 +202,18 @@ __device__ void hr_win_warp(const HrArgs& a, int i, int e_end, int plo, int phi,
     hr_wwalk_g(a.B + (int64_t)t * a.ldb, 1, t - 1 < phi ? t - 1 : phi, plo, a.rot, lane);
   }
 }
-// The factors of column jc on Q and Z, a warp each.
+// Pairs Jhi..Jlo of a column's factors on Q and Z, a warp each.
 __host__ __device__ int hr_qz_warps(const HrArgs& a) {
   const int rw = (a.n + 31) / 32;
   return (a.wantq ? (a.qrows ? a.n : rw) : 0) + (a.wantz ? rw : 0);
 }
-__device__ void hr_qz_warp(const HrArgs& a, int i, int jc, const double* rot, double* stage, int lane) {
+__device__ void hr_qz_warp(const HrArgs& a, int i, int Jhi, int Jlo, const double* rot, double* stage, int lane) {
   const int nq = a.wantq ? (a.qrows ? a.n : (a.n + 31) / 32) : 0;
   if (i < nq) {
-    if (a.qrows) hr_wwalk_g(a.Q + (int64_t)i * a.ldq, 1, a.ihi, jc + 2, rot, lane);
-    else hr_rows_item<true>(a.Q, a.ldq, 32 * i, a.n, a.ihi, jc + 2, rot, stage, lane);
+    if (a.qrows) hr_wwalk_g(a.Q + (int64_t)i * a.ldq, 1, Jhi, Jlo, rot, lane);
+    else hr_rows_item<true>(a.Q, a.ldq, 32 * i, a.n, Jhi, Jlo, rot, stage, lane);
   } else {
-    hr_rows_item<false>(a.Z, a.ldz, 32 * (i - nq), a.n, a.ihi, jc + 2, rot, stage, lane);
+    hr_rows_item<false>(a.Z, a.ldz, 32 * (i - nq), a.n, Jhi, Jlo, rot, stage, lane);
   }
 }
 
@@ -439,18 +439,22 @@ __device__ __forceinline__ void hr_window_cta(const HrArgs& a, int jc, int lo, i
 
 // Window (lo, hi) of column jc; (plo, phi): the previous window of the
 // column (plo < 0: none).  CTA 0 runs the window, the others the previous
-// window's walks, or the previous column's factors on Q and Z (its records:
-// prev; pjc < 0: none).
+// window's walks and, of the previous column's factors on Q and Z (its
+// records: prev; null: none), the pairs of this window's rows.  (All of them
+// in a column's first launch took 98 us of it at n = 2000, where a window
+// takes 39.)
 __global__ void __launch_bounds__(kHrThreads) k_hr_win(HrArgs a, int jc, int lo, int hi, int plo, int phi, int wmax,
-                                                       int pjc, const double* prev) {
+                                                       const double* prev) {
   extern __shared__ __align__(16) double sm[];
   if (blockIdx.x > 0) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n = gridDim.x - 1;
     double* const stage = sm + 2 * kHrStage * warp;
-    const int items = plo >= 0 ? hr_win_warps(a, lo - 1, plo) : hr_qz_warps(a);
+    const int wins = plo >= 0 ? hr_win_warps(a, lo - 1, plo) : 0, items = wins + (prev ? hr_qz_warps(a) : 0);
+    // column jc - 1 has one pair more, the topmost
+    const int qlo = lo == jc + 2 ? jc + 1 : lo;
     for (int i = (blockIdx.x - 1) + warp * n; i < items; i += n * kHrWarps) {
-      if (plo >= 0) hr_win_warp(a, i, lo - 1, plo, phi, stage, lane);
-      else hr_qz_warp(a, i, pjc, prev, stage, lane);
+      if (i < wins) hr_win_warp(a, i, lo - 1, plo, phi, stage, lane);
+      else hr_qz_warp(a, i - wins, hi, qlo, prev, stage, lane);
     }
     return;
   }
@@ -477,7 +481,7 @@ __global__ void __launch_bounds__(kHrThreads) k_hr_qz(HrArgs a, int jc) {
   __shared__ __align__(16) double stage[2 * kHrStage * kHrWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, items = hr_qz_warps(a);
   for (int i = blockIdx.x + warp * gridDim.x; i < items; i += gridDim.x * kHrWarps)
-    hr_qz_warp(a, i, jc, a.rot, stage + 2 * kHrStage * warp, lane);
+    hr_qz_warp(a, i, a.ihi, jc + 2, a.rot, stage + 2 * kHrStage * warp, lane);
 }
 
 int blocks_for(int items) { return std::max(1, (items + kHrThreads - 1) / kHrThreads); }
@@ -515,13 +519,13 @@ cudaError_t gghrd_device(cudaStream_t st, int icompq, int icompz, bool qrows, in
   const int qz = hr_qz_warps(a);
   for (int jc = ilo; jc <= ihi - 2 && e == cudaSuccess; ++jc) {
     a.rot = rot + 4 * (size_t)n * ((jc - ilo) & 1);
-    const double* prev = rot + 4 * (size_t)n * ((jc - ilo + 1) & 1);
+    const double* prev = jc > ilo ? rot + 4 * (size_t)n * ((jc - ilo + 1) & 1) : nullptr;
     int plo = -1, phi = -1;
     for (int hi = ihi; hi >= jc + 2;) {
       const int lo = hr_win_lo(jc, hi, W);
-      const int items = plo >= 0 ? hr_win_warps(a, lo - 1, plo) : jc > ilo ? qz : 0;
+      const int items = (plo >= 0 ? hr_win_warps(a, lo - 1, plo) : 0) + (prev ? qz : 0);
       const int helpers = std::min(items, std::max(1, sms - 1));
-      k_hr_win<<<1 + helpers, kHrThreads, smem, st>>>(a, jc, lo, hi, plo, phi, W, jc - 1, prev);
+      k_hr_win<<<1 + helpers, kHrThreads, smem, st>>>(a, jc, lo, hi, plo, phi, W, prev);
       ++launches;
       pairs += hi - lo + 1;
       plo = lo;
