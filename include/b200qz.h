@@ -177,8 +177,8 @@ int b200qz_mlp_train(float* params, const float* x, const float* target, int bat
 /* ------------------------------------------------------------------ */
 
 /* Reduce count independent pencils to generalized Schur form with Q, Z in
- * one persistent launch (CUDA-graph captured, replayed while the layout
- * stays the same).  Device buffers h, t, q, z hold pencil p (size n[p],
+ * persistent launches (CUDA-graph captured, replayed while the layout
+ * stays the same): one for the pencils above order 80, one for the rest.  Device buffers h, t, q, z hold pencil p (size n[p],
  * leading dimension n[p]) at offset moff[p] (in doubles); its eigenvalues
  * go to alphar/alphai/beta at offset eoff[p]; info[p] (device) is 0 or the
  * 1-based row that did not converge.  n, moff, eoff are host arrays.
