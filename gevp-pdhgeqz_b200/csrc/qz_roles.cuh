@@ -16,9 +16,13 @@
 // Warp 4 shares the core's scheduler and idles.  No barrier separates steps
 // or sweeps: the followers poll the core's step count, and the core waits
 // for the right warps once per sweep (before it reads rows they may still be
-// writing) and for everybody only when the ring is full.  Deflation tests
-// and shifts are the core's, from entries only the core writes, so they
-// overlap with the tail of the previous sweep.
+// writing) and for everybody only when the ring is full.  The deflation test
+// reads the diagonals and the subdiagonal, which only the core writes, and so
+// do the shifts of a block that ends where the last sweep ended (its final
+// step leaves rows l-1 and l to the core), so both overlap with the tail of
+// that sweep.  After a deflation at the bottom the block's last 2x2 lies
+// higher, and its entries H(l-1, l) and T(l-1, l) are the right warps': the
+// core waits for them before it forms the shift.
 //
 // Transformations are pairs of plane rotations formed with reciprocal
 // square roots.  Left: (a1, a2) -> (rho, 0), then (a0, rho) -> (beta, 0); both
@@ -529,6 +533,7 @@ __device__ int cta_role_qz(X& x, WinState& w, int maxit, RoleBuf* rb) {
     if (warp == 0) {
       RoleCore core{&w, rb, lane};
       int code = 0, a_if = 0, a_jz = -1;
+      int lswept = -1;  // last row of the latest sweep
       while (ilast >= 0) {
         // deflation: negligible subdiagonal, then zeros on T's diagonal
         bool dead = false;
@@ -572,6 +577,8 @@ __device__ int cta_role_qz(X& x, WinState& w, int maxit, RoleBuf* rb) {
         ++jiter;
         if (jiter > maxit) { code = 2; break; }
         const int l = ilast;
+        if (l != lswept && !role_wait_done(rb, kRoleRight, core.g, lane)) { code = 2; break; }
+        lswept = l;
         const double* h = Hb + (l - 1) + (l - 1) * ld;
         const double* t = Tb + (l - 1) + (l - 1) * ld;
         RoleCore::Shift p;

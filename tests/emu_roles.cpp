@@ -1,0 +1,102 @@
+// The window QZ with a role per warp (qz_roles.cuh), run as a thread block on
+// the host (warp_emu.h).  roles_host.inc is that header with its flag loads,
+// flag stores and predicated stores, which are PTX, left out: they are below.
+#include "warp_emu.h"
+
+#include <cfloat>
+
+#include "qz_window.cuh"
+namespace qz {
+inline int role_ld(const int* p) { return emu::polled(p); }
+inline void role_st(int* p, int v) {
+  *(volatile int*)p = v;
+  emu::posted();
+}
+inline unsigned role_sm(const void* p) { return (unsigned)((const char*)p - emu::block()->arena); }
+inline double* emu_at(unsigned a) { return (double*)(emu::block()->arena + a); }
+inline void role_put(bool on, unsigned a, double v) {
+  if (on) *emu_at(a) = v;
+}
+inline void role_put3(bool on, unsigned a, unsigned st, double v0, double v1, double v2) {
+  if (!on) return;
+  *emu_at(a) = v0;
+  *emu_at(a + st) = v1;
+  *emu_at(a + 2 * st) = v2;
+}
+inline void role_put8(bool on, unsigned a, double v0, double v1, double v2, double v3, double v4, double v5, double v6,
+                      double v7) {
+  const double v[8] = {v0, v1, v2, v3, v4, v5, v6, v7};
+  if (on) memcpy(emu_at(a), v, sizeof v);
+}
+inline void role_put_int2(bool on, unsigned a, int v0, int v1) {
+  const int v[2] = {v0, v1};
+  if (on) memcpy(emu_at(a), v, sizeof v);
+}
+inline void role_post(bool on, int* p, int v) {
+  if (on) role_st(p, v);
+}
+inline double role_rsqrt(double x) { return 1.0 / sqrt(x); }
+inline double role_rcp(double x) { return 1.0 / x; }
+}  // namespace qz
+#include "roles_host.inc"
+
+using namespace qz;
+
+namespace {
+struct EmuExec {
+  int tid, nt;
+  int* si;
+  double* sd;
+  void sync() { emu::block_barrier(); }
+  void stamp(int) {}
+  void count(int) {}
+};
+}  // namespace
+
+extern "C" {
+// Window QZ of (H, T) (n x n, in place), Q, Z its factors.  slow: warps that
+// run only when the others cannot get on.  Returns the status.
+int emu_role_qz(int n, double* H, double* T, double* Q, double* Z, unsigned slow) {
+  const int ld = n % 2 == 0 ? n + 1 : n;
+  std::vector<double> mem((size_t)4 * n * ld + kRoleDoubles + 3 * n + 8, 0.0);
+  double* const m = mem.data();
+  std::vector<int> si(64);
+  double hs = 0.0, ts = 0.0;
+  for (int j = 0; j < n; ++j)
+    for (int i = 0; i < n; ++i) {
+      hs += H[i + j * n] * H[i + j * n];
+      ts += T[i + j * n] * T[i + j * n];
+      m[i + j * ld] = H[i + j * n];
+      m[n * ld + i + j * ld] = T[i + j * n];
+      m[2 * n * ld + i + j * ld] = m[3 * n * ld + i + j * ld] = i == j ? 1.0 : 0.0;
+    }
+  RoleBuf* const rb = (RoleBuf*)(m + 4 * n * ld);
+  int status = -1;
+  emu::run(kRoleThreads, slow, (char*)m, [&](int tid) {
+    EmuExec x{tid, kRoleThreads, si.data(), (double*)(rb + 1)};
+    WinState w;
+    w.n = n;
+    w.H = MatV{m, ld};
+    w.T = MatV{m + n * ld, ld};
+    w.Q = MatV{m + 2 * n * ld, ld};
+    w.Z = MatV{m + 3 * n * ld, ld};
+    w.wantq = w.wantz = true;
+    w.tol.safmin = DBL_MIN;
+    w.tol.ulp = DBL_EPSILON;
+    w.tol.smlnum = DBL_MIN * ((double)n / DBL_EPSILON);
+    w.tol.htol = fmax(DBL_MIN, DBL_EPSILON * sqrt(hs));
+    w.tol.ttol = fmax(DBL_MIN, DBL_EPSILON * sqrt(ts));
+    const int r = cta_role_qz(x, w, 30 * n, rb);
+    if (r == 0) cta_std_all(x, w, x.sd);
+    if (tid == 0) status = r;
+  });
+  for (int j = 0; j < n; ++j)
+    for (int i = 0; i < n; ++i) {
+      H[i + j * n] = m[i + j * ld];
+      T[i + j * n] = m[n * ld + i + j * ld];
+      Q[i + j * n] = m[2 * n * ld + i + j * ld];
+      Z[i + j * n] = m[3 * n * ld + i + j * ld];
+    }
+  return status;
+}
+}

@@ -1,0 +1,195 @@
+// Device code of a thread block on one host thread: a fiber per CUDA thread.
+//
+// Warp collectives and block barriers are rendezvous of the fibers; flags in
+// "shared memory" are plain loads and stores, at which a fiber may be
+// switched out.  The order in which warps run is chosen by the test: every
+// warp in turn, or chosen warps only when no other can get on.  Code that
+// waits for what it reads gives the same bits under any order.
+#pragma once
+#include <ucontext.h>
+
+#include <cmath>
+#include <cstdint>
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <functional>
+#include <vector>
+
+namespace emu {
+
+constexpr int kLanes = 32;
+struct Fiber {
+  ucontext_t ctx;
+  std::vector<char> stack;
+  bool done = false;
+  bool waiting = false;  // at a rendezvous
+  uint64_t slot = 0;     // its contribution to a collective
+};
+struct Warp {
+  std::vector<uint64_t> vals = std::vector<uint64_t>(kLanes);
+  int arrived = 0;
+  long spins = 0;  // polls since the warp last saw a flag change or set one
+  const void* flag = nullptr;  // its latest poll
+  int value = 0;
+};
+
+struct Block {
+  std::vector<Fiber> f;
+  std::vector<Warp> w;
+  ucontext_t home;
+  int cur = 0, barrier = 0;
+  unsigned slow = 0;  // warps that run only when the others are stuck
+  std::function<void(int)> body;
+  char* arena = nullptr;  // "shared memory" (base of 32-bit addresses)
+};
+inline Block*& block() {
+  static Block* b = nullptr;
+  return b;
+}
+inline void yield() {
+  Block& b = *block();
+  swapcontext(&b.f[b.cur].ctx, &b.home);
+}
+inline int lane_id() { return block()->cur % kLanes; }
+
+// all lanes of the warp meet; returns the values they brought
+inline const std::vector<uint64_t>& meet(uint64_t v) {
+  Block& b = *block();
+  const int me = b.cur;
+  Warp& w = b.w[me / kLanes];
+  b.f[me].slot = v;
+  b.f[me].waiting = true;
+  if (++w.arrived == kLanes) {
+    w.arrived = 0;
+    const int base = me / kLanes * kLanes;
+    for (int i = 0; i < kLanes; ++i) {
+      w.vals[i] = b.f[base + i].slot;
+      b.f[base + i].waiting = false;
+    }
+    return w.vals;  // (nobody overwrites them before every lane has gone on to the next meeting)
+  }
+  while (b.f[me].waiting) yield();
+  return w.vals;
+}
+inline void block_barrier() {
+  Block& b = *block();
+  const int me = b.cur, total = (int)b.f.size();
+  b.f[me].waiting = true;
+  b.w[me / kLanes].spins = 0;
+  if (++b.barrier == total) {
+    b.barrier = 0;
+    for (Fiber& x : b.f) x.waiting = false;
+    return;
+  }
+  while (b.f[me].waiting) yield();
+}
+// a poll of a flag: the warp may be switched out
+inline int polled(const int* p) {
+  yield();
+  Warp& w = block()->w[block()->cur / kLanes];
+  const int v = *(const volatile int*)p;
+  if (w.flag == p && w.value != v) w.spins = 0;
+  w.flag = p;
+  w.value = v;
+  ++w.spins;
+  return v;
+}
+inline void posted() {
+  Block& b = *block();
+  b.w[b.cur / kLanes].spins = 0;
+}
+
+inline void entry(unsigned lo, unsigned hi) {
+  Block* b = (Block*)(((uintptr_t)hi << 32) | lo);
+  const int me = b->cur;
+  b->body(me);
+  b->f[me].done = true;
+  for (;;) yield();
+}
+
+// one turn of a warp: every lane that can run, until all have met or polled;
+// true if some lane was not just waiting
+inline bool turn(Block& b, int warp) {
+  bool ran = false;
+  for (int l = 0; l < kLanes; ++l) {
+    Fiber& x = b.f[warp * kLanes + l];
+    if (x.done || x.waiting) continue;
+    ran = true;
+    b.cur = warp * kLanes + l;
+    swapcontext(&b.home, &x.ctx);
+  }
+  return ran;
+}
+
+inline void run(int threads, unsigned slow, char* arena, const std::function<void(int)>& body) {
+  Block b;
+  b.f = std::vector<Fiber>(threads);
+  b.w = std::vector<Warp>(threads / kLanes);
+  b.slow = slow;
+  b.body = body;
+  b.arena = arena;
+  block() = &b;
+  for (Fiber& x : b.f) {
+    x.stack.resize(256 << 10);
+    getcontext(&x.ctx);
+    x.ctx.uc_stack.ss_sp = x.stack.data();
+    x.ctx.uc_stack.ss_size = x.stack.size();
+    x.ctx.uc_link = nullptr;
+    makecontext(&x.ctx, (void (*)())entry, 2, (unsigned)(uintptr_t)&b, (unsigned)((uintptr_t)&b >> 32));
+  }
+  const int warps = (int)b.w.size();
+  constexpr long kStuck = 8 * kLanes;  // polls in a row after which a warp counts as stuck
+  for (;;) {
+    bool left = false, on = false;
+    for (Fiber& x : b.f) left = left || !x.done;
+    if (!left) break;
+    for (int w = 0; w < warps; ++w)
+      if (!(slow >> w & 1)) on = (turn(b, w) && b.w[w].spins < kStuck) || on;
+    if (on) continue;
+    // nobody else gets on: the slow warps take a turn
+    for (int w = 0; w < warps; ++w)
+      if (slow >> w & 1) turn(b, w);
+  }
+  block() = nullptr;
+}
+
+}  // namespace emu
+
+// ---- the CUDA names the code uses ----
+#define __device__
+#define __host__
+#define __forceinline__ inline
+#define __noinline__
+struct double2 {
+  double x, y;
+};
+inline double2 make_double2(double x, double y) { return double2{x, y}; }
+inline uint64_t emu_bits(double v) {
+  uint64_t u;
+  memcpy(&u, &v, 8);
+  return u;
+}
+inline double emu_double(uint64_t u) {
+  double v;
+  memcpy(&v, &u, 8);
+  return v;
+}
+inline void __syncwarp() { emu::meet(0); }
+inline unsigned __ballot_sync(unsigned, bool p) {
+  const auto& v = emu::meet(p);
+  unsigned m = 0;
+  for (int i = 0; i < emu::kLanes; ++i) m |= (unsigned)(v[i] & 1) << i;
+  return m;
+}
+inline bool __all_sync(unsigned m, bool p) { return __ballot_sync(m, p) == 0xffffffffu; }
+inline bool __any_sync(unsigned m, bool p) { return __ballot_sync(m, p) != 0; }
+inline double __shfl_sync(unsigned, double v, int src) { return emu_double(emu::meet(emu_bits(v))[src & 31]); }
+inline int __shfl_sync(unsigned, int v, int src) { return (int)(uint32_t)emu::meet((uint32_t)v)[src & 31]; }
+inline double __shfl_up_sync(unsigned, double v, int d) {
+  const int l = emu::lane_id();
+  return emu_double(emu::meet(emu_bits(v))[l >= d ? l - d : l]);
+}
+inline double __shfl_xor_sync(unsigned, double v, int d) { return emu_double(emu::meet(emu_bits(v))[emu::lane_id() ^ d]); }
+inline int __ffs(unsigned v) { return __builtin_ffs((int)v); }
+inline int __double2hiint(double v) { return (int)(emu_bits(v) >> 32); }
