@@ -197,12 +197,17 @@ __device__ __forceinline__ void role_apply_right(double cb, double sb, double cc
   x0 = cc * x0 - sc * d;
 }
 
-// wait until every flag of the mask (bit w: done[w]) is at least v
+// wait until every flag of the mask (bit w: done[w]) is at least v (a vote
+// orders no memory: the lanes that polled nothing get the pollers' acquire
+// from the warp barrier)
 __device__ __forceinline__ bool role_wait_done(RoleBuf* rb, unsigned mask, int v, int lane) {
   const bool mine = lane < 8 && ((mask >> lane) & 1);
   for (int it = 0; it < kRoleSpin; ++it) {
     const bool ok = !mine || role_ld(&rb->done[lane & 7]) >= v;
-    if (__all_sync(0xffffffffu, ok)) return true;
+    if (__all_sync(0xffffffffu, ok)) {
+      __syncwarp();
+      return true;
+    }
   }
   if (lane == 0) role_st(&rb->err, 1);
   __syncwarp();

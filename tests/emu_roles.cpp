@@ -99,4 +99,29 @@ int emu_role_qz(int n, double* H, double* T, double* Q, double* Z, unsigned slow
     }
   return status;
 }
+
+// role_wait_done by warp 0 while warps 1 and 2 post their counts up to v:
+// lanes of warp 0 whose later reads are ordered behind both counts.
+int emu_wait_done(int v) {
+  std::vector<double> mem(kRoleDoubles, 0.0);
+  RoleBuf* const rb = (RoleBuf*)mem.data();
+  int lanes = 0;
+  emu::run(
+      96, 0, (char*)mem.data(),
+      [&](int tid) {
+        const int warp = tid / 32, lane = tid % 32;
+        if (warp != 0) {
+          for (int k = 1; k <= v; ++k) {
+            __syncwarp();
+            if (lane == 0) role_st(&rb->done[warp], k);
+          }
+          return;
+        }
+        if (!role_wait_done(rb, kRoleRight, v, lane)) return;
+        auto& s = emu::block()->seen[tid];
+        if (s[&rb->done[1]] >= v && s[&rb->done[2]] >= v) ++lanes;
+      },
+      true);
+  return lanes;
+}
 }

@@ -78,3 +78,9 @@ def test_any_order_of_the_warps(emu, lapack, n, kind, seed):
         assert rc == 0, slow
         for k, (a, b) in enumerate(zip(first, out)):
             assert np.array_equal(a.view(np.int64), b.view(np.int64)), (slow, k, np.abs(a - b).max())
+
+
+def test_wait_orders_every_lane(emu):
+    """Only some lanes poll the counts that a wait is for, but all of them read
+    what the counts stand for: each lane has to be ordered behind the polls."""
+    assert emu.emu_wait_done(7) == 32

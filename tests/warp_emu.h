@@ -14,6 +14,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <functional>
+#include <map>
 #include <vector>
 
 namespace emu {
@@ -42,6 +43,11 @@ struct Block {
   unsigned slow = 0;  // warps that run only when the others are stuck
   std::function<void(int)> body;
   char* arena = nullptr;  // "shared memory" (base of 32-bit addresses)
+  // With ordered set: the largest value of every flag that each thread's later
+  // reads are ordered behind, by a poll of its own or by a warp barrier after
+  // another lane's (a vote hands nothing over).
+  bool ordered = false;
+  std::vector<std::map<const void*, int>> seen;
 };
 inline Block*& block() {
   static Block* b = nullptr;
@@ -93,6 +99,10 @@ inline int polled(const int* p) {
   w.flag = p;
   w.value = v;
   ++w.spins;
+  if (block()->ordered) {
+    int& s = block()->seen[block()->cur][p];
+    s = s > v ? s : v;
+  }
   return v;
 }
 inline void posted() {
@@ -122,8 +132,10 @@ inline bool turn(Block& b, int warp) {
   return ran;
 }
 
-inline void run(int threads, unsigned slow, char* arena, const std::function<void(int)>& body) {
+inline void run(int threads, unsigned slow, char* arena, const std::function<void(int)>& body, bool ordered = false) {
   Block b;
+  b.ordered = ordered;
+  b.seen.resize(threads);
   b.f = std::vector<Fiber>(threads);
   b.w = std::vector<Warp>(threads / kLanes);
   b.slow = slow;
@@ -175,7 +187,17 @@ inline double emu_double(uint64_t u) {
   memcpy(&v, &u, 8);
   return v;
 }
-inline void __syncwarp() { emu::meet(0); }
+inline void __syncwarp() {
+  emu::meet(0);
+  emu::Block& b = *emu::block();
+  if (!b.ordered) return;
+  const int base = b.cur / emu::kLanes * emu::kLanes;
+  for (int i = base; i < base + emu::kLanes; ++i)
+    for (const auto& s : b.seen[i]) {
+      int& mine = b.seen[b.cur][s.first];
+      mine = mine > s.second ? mine : s.second;
+    }
+}
 inline unsigned __ballot_sync(unsigned, bool p) {
   const auto& v = emu::meet(p);
   unsigned m = 0;
