@@ -491,7 +491,11 @@ __device__ inline void role_follow(WinState& w, RoleBuf* rb, int warp, int lane)
         break;
       }
     }
-    if (!__any_sync(0xffffffffu, go)) return;
+    if (!__any_sync(0xffffffffu, go)) {
+      // the end, unless the wait gave up: steps would be lost then
+      if (lane == 0 && (role_ld(&rb->stop) == 0 || role_ld(&rb->ready) > g)) role_st(&rb->err, 1);
+      return;
+    }
     __syncwarp();
     const double* sl = rb->ring[g & (kRoleRing - 1)];
     const int s = ((const int*)(sl + 8))[0];
@@ -524,7 +528,8 @@ __device__ inline void role_follow(WinState& w, RoleBuf* rb, int warp, int lane)
 }
 
 // Window QZ of a window in shared memory by kRoleThreads threads: 0, or
-// ilast+1 if it did not converge.  The 2x2 blocks stay general.
+// ilast+1 (at least 1) if it did not converge or a wait gave up.  The 2x2
+// blocks stay general.
 template <class X>
 __device__ int cta_role_qz(X& x, WinState& w, int maxit, RoleBuf* rb) {
   const int n = w.n, ld = w.H.ld, lane = x.tid & 31, warp = x.tid >> 5;
@@ -610,7 +615,8 @@ __device__ int cta_role_qz(X& x, WinState& w, int maxit, RoleBuf* rb) {
     x.sync();
     const int code = rb->code, f = rb->arg[0], jz = rb->arg[1], il = rb->arg[2], err = rb->err;
     x.sync();
-    if (err != 0 || code == 2) return il + 1;
+    // (a follower may give up when the core is past its last row)
+    if (err != 0 || code == 2) return il >= 0 ? il + 1 : 1;
     if (code == 0) return 0;
     // a zero on T's diagonal: infinite eigenvalue, all threads
     if (jz == f) {

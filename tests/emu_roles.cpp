@@ -55,8 +55,10 @@ struct EmuExec {
 
 extern "C" {
 // Window QZ of (H, T) (n x n, in place), Q, Z its factors.  slow: warps that
-// run only when the others cannot get on.  Returns the status.
-int emu_role_qz(int n, double* H, double* T, double* Q, double* Z, unsigned slow) {
+// run only when the others cannot get on; spin: polls before a wait gives up.
+// Returns the status.
+int emu_role_qz(int n, double* H, double* T, double* Q, double* Z, unsigned slow, int spin) {
+  kRoleSpin = spin;
   const int ld = n % 2 == 0 ? n + 1 : n;
   std::vector<double> mem((size_t)4 * n * ld + kRoleDoubles + 3 * n + 8, 0.0);
   double* const m = mem.data();
@@ -103,6 +105,7 @@ int emu_role_qz(int n, double* H, double* T, double* Q, double* Z, unsigned slow
 // role_wait_done by warp 0 while warps 1 and 2 post their counts up to v:
 // lanes of warp 0 whose later reads are ordered behind both counts.
 int emu_wait_done(int v) {
+  kRoleSpin = 1 << 22;
   std::vector<double> mem(kRoleDoubles, 0.0);
   RoleBuf* const rb = (RoleBuf*)mem.data();
   int lanes = 0;
