@@ -402,7 +402,8 @@ __device__ inline int big_solve(const BigPencil& p, double* smem, int maxit) {
       __syncthreads();
       const int mu = sh->si[8], status = sh->si[9], changed = sh->si[10];
       if (status == 0 && changed) {
-        if (!whole && tid == 0) p.H[kwtop + (size_t)(kwtop - 1) * n] = s * Us[0];
+        // (as k_aed_win stores it)
+        if (!whole && tid == 0) p.H[kwtop + (size_t)(kwtop - 1) * n] = mu > 0 ? s * Us[0] : 0.0;
         big_store(p, kwtop, nw, Hs, Ts, ld);
         big_update(p, kwtop, nw, Us, Vs, ld, big_slab(m, 4 * nw * ld));
       }

@@ -141,7 +141,9 @@ __global__ void __launch_bounds__(kThreads) k_aed_win(double* H, double* T, int6
         Zw[idx] = Zs[i + j * lw];
       }
     }
-    if (threadIdx.x == 0 && kwtop > ktop) G(H, ld, kwtop, kwtop - 1) = s * Qs[0];
+    // the spike's first entry; negligible, and zero, when the whole window
+    // deflated
+    if (threadIdx.x == 0 && kwtop > ktop) G(H, ld, kwtop, kwtop - 1) = m > 0 ? s * Qs[0] : 0.0;
   }
   if (threadIdx.x == 0) {
     info[0] = m;
