@@ -287,9 +287,32 @@ struct NoAllocDev {
 NoAllocDev g_noalloc_dev[kNoAllocMaxDevices];
 std::mutex g_noalloc_mu;
 
+// Both kernels on an empty queue, waited for.  k_batch_big's frame (its rare
+// block swaps in doubled precision, at 128 registers) is larger than the
+// per-thread stack a context begins with, and CUDA takes the device memory for
+// a larger one, about 78 MB, at the first launch that needs it.
+cudaError_t noalloc_first_launches(int* counter) {
+  cudaStream_t st;
+  cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+  if (e != cudaSuccess) return e;
+  int none = 0, smem_max = kBatchSmemMax;
+  const int* ip = nullptr;
+  const int64_t* lp = nullptr;
+  double* dp = nullptr;
+  int* status = nullptr;
+  // (as launch_batch passes them)
+  void* args[] = {&none, &ip, &ip, &lp, &lp, &dp, &dp, &dp, &dp, &dp, &dp, &dp, &status, &counter, &smem_max};
+  e = cudaLaunchKernel((const void*)k_batch_big, dim3(1), dim3(kBigThreads), args, kBigSmem, st);
+  if (e == cudaSuccess)
+    e = cudaLaunchKernel((const void*)k_batch_qz, dim3(1), dim3(kRoleThreads), args, batch_smem_bytes(smem_max), st);
+  const cudaError_t es = cudaStreamSynchronize(st), ed = cudaStreamDestroy(st);
+  return e != cudaSuccess ? e : es != cudaSuccess ? es : ed;
+}
+
 // Once per device, with that device current: the device address of the
-// scratch array (its host-side name is only a stand-in), the SM count and
-// the kernel's shared-memory limit.
+// scratch array (its host-side name is only a stand-in), the SM count, the
+// kernels' shared-memory limits and their first launches, so that no later
+// call has to take device memory.
 int noalloc_setup(int dev, NoAllocDev** out) {
   if (dev < 0 || dev >= kNoAllocMaxDevices) return 10001;
   std::lock_guard<std::mutex> lk(g_noalloc_mu);
@@ -299,6 +322,7 @@ int noalloc_setup(int dev, NoAllocDev** out) {
     if (cudaGetSymbolAddress(&p, g_noalloc_scratch) != cudaSuccess) return 10001;
     if (cudaDeviceGetAttribute(&d.sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 10001;
     if (batch_init() != cudaSuccess) return 10001;
+    if (noalloc_first_launches((int*)((unsigned char*)p + kNoAllocBytes - 256)) != cudaSuccess) return 10001;
     d.scratch = (unsigned char*)p;
     d.ready = true;
   }

@@ -217,12 +217,14 @@ int b200qz_batched_config(const b200qz_ctx* ctx, int* threads, int* smem_max, in
  * library's device memory (about 96 KB, held by every GPU that loads the
  * library until the process exits), so at most 4096 pencils per call: a
  * larger count returns -2.  The first call on a device sets that device up
- * (it looks up the array's device address and raises the kernel's shared-
- * memory limit), so make it before any stream capture.  All calls share
- * the array: calls whose work overlaps on the GPU (different streams, or
- * host threads racing) corrupt each other's batches.  Returns 0, -1 bad
- * count, -2 count above 4096, -3 a size outside 1..46340, or 10001 on a
- * CUDA error of this call.  No counterpart in the reference. */
+ * (it looks up the array's device address, raises the kernels' shared-memory
+ * limits and launches them once on no pencils, which is when CUDA takes the
+ * memory for their per-thread stack), whatever its pencils, and waits for
+ * that; make it before any stream capture.  Later calls take no device
+ * memory.  All calls share the array: calls whose work overlaps on the GPU
+ * (different streams, or host threads racing) corrupt each other's batches.
+ * Returns 0, -1 bad count, -2 count above 4096, -3 a size outside 1..46340,
+ * or 10001 on a CUDA error of this call.  No counterpart in the reference. */
 int b200qz_solve_batched_noalloc(int count, const int* n, const long long* moff, const long long* eoff,
                                  double* h, double* t, double* q, double* z, double* alphar, double* alphai,
                                  double* beta, int* info, void* stream);
