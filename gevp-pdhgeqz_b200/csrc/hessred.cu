@@ -432,7 +432,16 @@ __device__ __forceinline__ void hr_window_cta(const HrArgs& a, int jc, int lo, i
   __syncthreads();
   if (warp < groups) hr_chain_warp(L, m, ldw, warp, w, lane, a.err);
   __syncthreads();
-  for (int i = 4 + tid; i < 4 * m; i += kHrThreads) a.rot[4 * (int64_t)o + i] = L.gbuf[i];
+  // The records, normed to first order: c and s of a pair are rounded
+  // separately, c^2 + s^2 is off by 1.2 units of rounding (root mean square;
+  // 0.65 so), and every pair multiplies that into whole rows of Q and Z.
+  for (int i = 2 + tid; i < 2 * m; i += kHrThreads) {
+    double2 r = ((const double2*)L.gbuf)[i];
+    const double h = 0.5 * fma(-r.y, r.y, fma(-r.x, r.x, 1.0));
+    r.x = fma(r.x, h, r.x);
+    r.y = fma(r.y, h, r.y);
+    ((double2*)(a.rot + 4 * (int64_t)o))[i] = r;
+  }
   for (int j = warp; j < m; j += kHrWarps)
     for (int i = lane; i <= j; i += 32) Bo[i + (int64_t)j * a.ldb] = L.Tw[i + j * ldw];
 }
