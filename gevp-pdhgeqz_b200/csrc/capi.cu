@@ -637,13 +637,13 @@ int b200qz_set_params(b200qz_ctx* c, int nw_max, int w_chase, int nmin, int nibb
   if (w_chase > kWinSmemMax || (w_chase >= 0 && w_chase < 12)) return -3;
   if (nmin > kAedMax) return -4;
   if (nibble > 100) return -5;
-  if (nw_max >= 0) c->params.nw_max = std::max(4, nw_max);
+  if (nw_max >= 0) c->params.nw_max = nw_max == 0 ? 0 : std::max(4, nw_max);  // 0: by order
   if (w_chase >= 0) c->params.w_chase = w_chase;
   if (nmin >= 0) c->params.nmin = std::max(4, nmin);
   if (nibble >= 0) c->params.nibble = nibble;
   if (ns_max >= 0) c->params.ns_max = ns_max;
   if (maxit_factor >= 0) c->params.maxit_factor = std::max(1, maxit_factor);
-  if (w_chase >= 0) c->params.chain_max = std::min(kMaxChain, std::max(1, (c->params.w_chase - 4) / 6));
+  if (w_chase >= 0) c->params.chain_max = std::min(kMaxChain, chain_of_window(w_chase));
   return 0;
 }
 
@@ -652,9 +652,9 @@ int b200qz_set_param(b200qz_ctx* c, const char* name, double value) {
   std::string k(name);
   int v = (int)value;
   SolveParams& P = c->params;
-  if (k == "nw_max") { if (v < 4 || v > kWinSmemMax) return -3; P.nw_max = v; }
+  if (k == "nw_max") { if (v != 0 && (v < 4 || v > kWinSmemMax)) return -3; P.nw_max = v; }
   else if (k == "w_chase") { if (v < 12 || v > kWinSmemMax) return -3; P.w_chase = v;
-    P.chain_max = std::min(kMaxChain, std::max(1, (v - 4) / 6)); }
+    P.chain_max = std::min(kMaxChain, chain_of_window(v)); }
   else if (k == "nmin") { if (v < 4 || v > kAedMax) return -3; P.nmin = v; }
   else if (k == "nibble") { if (v < 0 || v > 100) return -3; P.nibble = v; }
   else if (k == "ns_max") { if (v < 0) return -3; P.ns_max = v; }

@@ -19,11 +19,19 @@
 
 namespace qz {
 
+// Default chase window and bulges per chain (SolveParams::w_chase).
+constexpr int kChaseWindow = 64, kChaseChain = 8;
+// Bulges per chain of a chase window that a caller chooses: half of the window
+// is left to advance in.  The default window keeps its own chain, a bulge per
+// chase warp (n=1800 278 ms with 8 and 291 with 10, n=901 102 and 111; a window
+// of 80 is as fast with 12 as with 8: 312 and 325, 129 and 122).
+inline int chain_of_window(int w) { return w == kChaseWindow ? kChaseChain : std::max(1, (w - 4) / 6); }
+
 // Tunables (defaults follow the reference's PIPARMQ table where the GPU
 // window limits allow; see piparmq.f:438-535).
 struct SolveParams {
   int nw_max = 0;        // AED window (one CTA, shared memory; up to 80); 0: table
-  int w_chase = 64;      // chase window and bulges per chain: 64 and 8 (a bulge per
+  int w_chase = kChaseWindow;  // chase window and bulges per chain: 64 and 8 (a bulge per
                          // chase warp).  A step of the chase kernel costs 2,270
                          // cycles there and 4,340 for 12 bulges in 80 rows, and the
                          // shorter chains of a sweep run on more SMs at once:
@@ -33,7 +41,7 @@ struct SolveParams {
   int nibble = -1;       // -1: table (nibble_table)
   int ns_max = -1;       // -1: table
   int maxit_factor = 30; // MAXIT = 30*NH
-  int chain_max = 8;     // -1: from w_chase
+  int chain_max = kChaseChain;  // -1: from w_chase
   int verbose = 0;       // progress lines on stderr (B200QZ_VERBOSE=1)
   int aed_nskip = -1;    // AED spike test stops after this many consecutive
                          // undeflatable blocks (0: test the whole window;

@@ -111,16 +111,19 @@ int b200qz_solve_host(b200qz_ctx* ctx, char job, char compq, char compz, int n, 
  * Returns the number of values written. */
 int b200qz_get_stats(const b200qz_ctx* ctx, double* out, int nout);
 
-/* Tunables: nw_max (AED window), w_chase (chase window), nmin (blocks
- * solved by one CTA), nibble (percent), ns_max (shift cap), maxit factor.
+/* Tunables: nw_max (AED window; 0, the default: by the pencil's order),
+ * w_chase (chase window; sets the bulges per chain with it), nmin (blocks
+ * solved by one CTA), nibble (percent), ns_max (shift cap; 0: by the active
+ * block's order), maxit factor.
  * A value < 0 keeps the current setting. Returns 0 or -i for argument i. */
 int b200qz_set_params(b200qz_ctx* ctx, int nw_max, int w_chase, int nmin, int nibble, int ns_max,
                       int maxit_factor);
 
 /* Set one tunable by name: "nw_max", "w_chase", "nmin", "nibble",
- * "ns_max", "maxit_factor", "chain_max" (bulges per chain), "aed_nskip"
- * (AED spike test stops after this many consecutive undeflatable blocks,
- * 0 = whole window), "max_wave" (chains chased concurrently, 1..8),
+ * "ns_max", "maxit_factor" (as above), "chain_max" (bulges per chain; set by
+ * "w_chase" too), "aed_nskip" (AED spike test stops after this many
+ * consecutive undeflatable blocks, 0 = whole window, -1, the default: by the
+ * pencil's order), "max_wave" (chains chased concurrently, 1..8),
  * "stall_limit" (iterations without deflation before INFO > 0),
  * "split" (0, 7 or 8 INT8 Ozaki slices for the off-diagonal updates),
  * "aed_threads" (32, 64, 128 or 256), "upd_persist" (0 or 1), "aed_limit"
