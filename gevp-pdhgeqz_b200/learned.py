@@ -40,7 +40,7 @@ TRACES = os.path.join(POLICY_DIR, "traces.npz")
 
 NIN, NHID, NOUT = 64, 128, 2
 NW_MIN, NW_SPAN, NW_MAX = 16, 64, 80
-TABLE_NW = 48  # the fixed AED window the policy is compared with
+TABLE_NW = 48  # the fixed AED window of traces recorded before the window went by order
 GRID_NW = (24, 32, 40, 48, 56, 64, 80)
 GRID_NSF = (0.5, 1.0)
 DECISIONS = (0, 5, 20, 60, 150)  # AED indices at which a trace samples the choice
@@ -154,8 +154,15 @@ def encode(nw: int, nsf: float):
     return np.array([(nw - NW_MIN) / NW_SPAN, nsf], dtype=np.float32)
 
 
+def table_window(n: int) -> int:
+    """The solver's AED window for a pencil of order n (nw_table in
+    csrc/qz_solver.h)."""
+    return 24 if n < 600 else 32 if n < 1200 else 48 if n < 3000 else 56
+
+
 def table_choice(nh: int, table_nw: int = TABLE_NW):
-    """(nw, ns/nw) the fixed table gives (nw_max and NS(NH), piparmq.f:504-533)."""
+    """(nw, ns/nw) the fixed table gives for an active block of order nh: the
+    AED window table_nw and NS(NH) (piparmq.f:504-533)."""
     ns = 2
     if nh >= 30:
         ns = 4
@@ -222,7 +229,8 @@ def _solve(solver, bufs, n):
 
 
 def _set(solver, nw_max, ns_max, aed_limit):
-    """ns_max 0: the table's NS(NH); aed_limit -1: no limit."""
+    """nw_max 0: the table's window; ns_max 0: the table's NS(NH); aed_limit
+    -1: no limit."""
     solver.set_param("nw_max", nw_max)
     solver.set_param("ns_max", ns_max)
     solver.set_param("aed_limit", aed_limit)
@@ -244,7 +252,7 @@ def trace_pencil(solver, H, T, decisions=DECISIONS, horizon=3):
     for j in decisions:
         bufs[0].copy_(dH0)
         bufs[1].copy_(dT0)
-        _set(solver, TABLE_NW, 0, j)
+        _set(solver, 0, 0, j)
         info = _solve(solver, bufs, n)
         st = solver.stats()
         if info != 10003:
@@ -258,7 +266,7 @@ def trace_pencil(solver, H, T, decisions=DECISIONS, horizon=3):
         # cost of restarting from the snapshot alone (scans down to kbot)
         bufs[0].copy_(snapH)
         bufs[1].copy_(snapT)
-        _set(solver, TABLE_NW, 0, 0)
+        _set(solver, 0, 0, 0)
         _solve(solver, bufs, n)
         t0 = solver.stats()["seconds"]
         s_time = np.zeros((len(GRID_NW), len(GRID_NSF)))
@@ -278,7 +286,7 @@ def trace_pencil(solver, H, T, decisions=DECISIONS, horizon=3):
                 s_flop[a, b] = defl / max(cost, 1.0)
                 s_time[a, b] = defl / max(st["seconds"] - t0, 1e-6)
         out.append((feat, s_time, s_flop, kbot - ktop + 1))
-    _set(solver, TABLE_NW, 0, -1)
+    _set(solver, 0, 0, -1)
     return out
 
 
@@ -298,9 +306,12 @@ def score_of_choice(score, nw, nsf, grid_nw=GRID_NW, grid_nsf=GRID_NSF):
 
 def trace_grid(tr):
     """(grid_nw, grid_nsf, table_nw) a trace file was recorded with (files
-    without them predate the current grid)."""
+    without them predate the current grid).  table_nw is one window, or an
+    array with the window of every sample."""
     if "grid_nw" in tr:
-        return tuple(int(v) for v in tr["grid_nw"]), tuple(float(v) for v in tr["grid_nsf"]), int(tr["table_nw"])
+        tnw = np.asarray(tr["table_nw"])
+        return (tuple(int(v) for v in tr["grid_nw"]), tuple(float(v) for v in tr["grid_nsf"]),
+                int(tnw) if tnw.ndim == 0 else tnw)
     return (24, 40, 56, 80), (0.5, 1.0), 80
 
 
@@ -308,13 +319,15 @@ def offline_gain(P, X, scores, nh, grid=None):
     """Geometric mean over samples of score(network's choice) /
     score(table's choice), both taken at the nearest grid candidate (ratios
     floored at 1e-3 so that a zero score counts as a large loss, not -inf).
-    grid: (grid_nw, grid_nsf, table_nw) of the traces (trace_grid)."""
+    grid: (grid_nw, grid_nsf, table_nw) of the traces (trace_grid), an array
+    table_nw with an entry per sample."""
     gnw, gnsf, tnw_fixed = grid if grid is not None else (GRID_NW, GRID_NSF, TABLE_NW)
+    windows = np.broadcast_to(tnw_fixed, len(nh))
     _, _, Y = forward_np(P, X)
     logs = []
-    for y, sc, h in zip(Y, scores, nh):
+    for y, sc, h, window in zip(Y, scores, nh, windows):
         nw, ns = decode(y, int(h))
-        tnw, tnsf = table_choice(int(h), tnw_fixed)
+        tnw, tnsf = table_choice(int(h), int(window))
         s_net = score_of_choice(sc, nw, ns / max(nw, 1), gnw, gnsf)
         s_tab = score_of_choice(sc, tnw, tnsf, gnw, gnsf)
         if s_tab > 0:
@@ -328,7 +341,7 @@ def generate_traces(count=200, decisions=DECISIONS, device=0, log=None):
     pkg = _pkg()
     torch.cuda.set_device(device)
     solver = pkg.Solver(device)
-    feats, scores, sflop, nhs, ids = [], [], [], [], []
+    feats, scores, sflop, nhs, ids, windows = [], [], [], [], [], []
     try:
         for i, n, seed in training_pencils(count):
             H, T = pkg.pencils.clustered_ht(n, seed, every=50, scale=1e-8)
@@ -338,11 +351,12 @@ def generate_traces(count=200, decisions=DECISIONS, device=0, log=None):
                 sflop.append(sf)
                 nhs.append(nh)
                 ids.append(i)
+                windows.append(table_window(n))
             if log:
                 log("pencil %d n=%d samples=%d" % (i, n, len(feats)))
     finally:
         solver.close()
     return {"features": np.stack(feats).astype(np.float32), "scores": np.stack(scores),
             "scores_per_flop": np.stack(sflop), "nh": np.array(nhs), "pencil": np.array(ids),
-            "grid_nw": np.array(GRID_NW), "grid_nsf": np.array(GRID_NSF), "table_nw": TABLE_NW,
+            "grid_nw": np.array(GRID_NW), "grid_nsf": np.array(GRID_NSF), "table_nw": np.array(windows),
             "decisions": np.array(decisions)}

@@ -59,6 +59,10 @@ def cmd_train(a):
     grid = lrn.trace_grid(tr)
     T = lrn.labels_from_scores(scores, grid[0], grid[1])
     hold = pid % 5 == 0
+
+    def part(mask):  # the grid of a part of the samples
+        return grid[0], grid[1], grid[2][mask] if np.ndim(grid[2]) else grid[2]
+
     P0 = lrn.init_params(a.seed)
     t0 = time.time()
     P, mse = lrn.train_device(P0, X[~hold], T[~hold], epochs=a.epochs, lr=a.lr)
@@ -66,8 +70,8 @@ def cmd_train(a):
     res = {"samples_train": int((~hold).sum()), "samples_holdout": int(hold.sum()), "mse_train": mse,
            "label": "argmax deflations per device second",
            "mse_holdout": lrn.loss_np(P, X[hold], T[hold]), "train_seconds": dt,
-           "gain_train": lrn.offline_gain(P, X[~hold], scores[~hold], nh[~hold], grid),
-           "gain_holdout": lrn.offline_gain(P, X[hold], scores[hold], nh[hold], grid)}
+           "gain_train": lrn.offline_gain(P, X[~hold], scores[~hold], nh[~hold], part(~hold)),
+           "gain_holdout": lrn.offline_gain(P, X[hold], scores[hold], nh[hold], part(hold))}
     os.makedirs(a.out, exist_ok=True)
     np.savez_compressed(os.path.join(a.out, "weights.npz"), params=P, epochs=a.epochs, lr=a.lr, seed=a.seed)
     print(json.dumps(res), flush=True)

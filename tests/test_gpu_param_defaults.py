@@ -79,3 +79,15 @@ def test_out_of_range_stays_refused(pkg):
             s.set_params(nw_max=81)
     finally:
         s.close()
+
+
+def test_trace_leaves_the_solver_as_it_was(pkg, fresh):
+    H, T, want, counts = fresh
+
+    def trace(s):
+        Ht, Tt = pkg.pencils.clustered_ht(300, 5)
+        assert len(pkg.learned.trace_pencil(s, Ht, Tt, decisions=(0,), horizon=1)) == 1
+
+    out, got = _solve(pkg, H, T, trace)
+    assert got == counts
+    assert all(torch.equal(a, b) for a, b in zip(want, out))
