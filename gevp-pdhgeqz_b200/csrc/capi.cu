@@ -166,6 +166,7 @@ struct GpuBackend {
   double *H, *T, *Q, *Z;
   int64_t ld;
   int n;
+  int nh0;  // order of the block the solve began with (ihi - ilo + 1)
   bool wantq, wantz;
   // JOB = 'S': full Schur form.  JOB = 'E' (eigenvalues only): the far
   // updates of H and T stop at the active block [act_top, act_bot], the
@@ -195,14 +196,10 @@ struct GpuBackend {
     if (c->err != cudaSuccess) { out[0] = ifirst; out[1] = 0; out[2] = -1; out[3] = -1; out[4] = 1; return; }
     for (int i = 0; i < 5; ++i) out[i] = c->hinfo[i];
   }
-  // Consecutive undeflatable blocks after which the spike test stops (0: the
-  // whole window).  Automatic: the whole window for pencils of order 900 and
-  // more (n=1800: 387 against 410 ms stopping after 4, n=901 145 against
-  // 148), 4 below, where a window's moves cost more than the sweeps they save
-  // (n=700 123 against 130, n=201 30 against 38).
+  // consecutive undeflatable blocks after which the spike test stops
   int aed_early_stop() const {
     if (c->params.aed_nskip >= 0) return c->params.aed_nskip;
-    return n >= 900 ? 0 : 4;
+    return nskip_table(nh0);
   }
   void aed(int ktop, int kwtop, int kbot, int* info3, double* sh) {
     int nw = kbot - kwtop + 1;
@@ -521,6 +518,7 @@ int solve_dev_impl(b200qz_ctx* c, char job, char compq, char compz, int n, int i
   bk.H = h; bk.T = t; bk.Q = q; bk.Z = z;
   bk.ld = ld;
   bk.n = n;
+  bk.nh0 = nh;
   bk.wantq = wantq;
   bk.wantz = wantz;
   bk.schur = is(job, 'S');

@@ -45,7 +45,7 @@ struct SolveParams {
   int verbose = 0;       // progress lines on stderr (B200QZ_VERBOSE=1)
   int aed_nskip = -1;    // AED spike test stops after this many consecutive
                          // undeflatable blocks (0: test the whole window;
-                         // -1: whole window for n >= 900, else 4)
+                         // -1: nskip_table)
   int max_wave = 8;      // chains chased concurrently (one CTA each)
   int stall_limit = 300; // iterations without deflation before giving up
   int aed_threads = 256; // threads of the AED / endgame window kernel (256: a role
@@ -115,6 +115,16 @@ inline int nw_table(int nh) {
   if (nh < 3000) return 48;
   return 56;
 }
+
+// Consecutive undeflatable blocks after which the spike test stops, for a
+// pencil of order nh (0: the whole window).  Below the line a window's moves
+// cost more than the sweeps they save.  Time with the whole window over the
+// time with 4, means of four pencils at n = 300 / 500 / 600 / 700 / 800 / 901:
+// Hessenberg-triangular forms of dense pairs 1.07 / 1.02 / 1.00 / 1.01 / 0.99 /
+// 0.96, with 5 % infinite eigenvalues 1.10 / 0.99 / 1.04 / 1.02 / 0.98 / 1.00,
+// graded 1.03 / 1.03 / 1.01 / 1.02 / 0.99 / 0.98 (N(0,1) entries in T, where
+// much deflates early: 0.95 / 0.94 / 0.93 / 0.90 / 0.91 / 0.88).
+inline int nskip_table(int nh) { return nh >= 750 ? 0 : 4; }
 
 // Power of two applied to T before the iteration when T's magnitude is far
 // from H's (more than 2^30 apart), so that shift polynomials, whose
