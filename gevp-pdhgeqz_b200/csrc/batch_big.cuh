@@ -12,6 +12,7 @@
 // L2), and the chases, 22 % (115k cycles each: a serial chain of reflectors).
 #pragma once
 #include "qz_chase_roles.cuh"
+#include "qz_solver.h"
 #include "update.cuh"
 
 namespace qz {
@@ -344,7 +345,7 @@ __device__ inline int big_solve(const BigPencil& p, double* smem, int maxit) {
   const BigMem m = big_mem(smem);
   BigShare* const sh = m.sh;
   const int tid = threadIdx.x, n = p.n;
-  const int nw_aed = n < 600 ? 24 : n < 1200 ? 32 : 48;  // nw_table
+  const int nw_aed = nw_table(n);
   int ifirst = 0, kbot = n - 1, stall = 0, last_kbot = -1, last_ktop = -1;
   for (int it = 0; it < maxit; ++it) {
     if (kbot < ifirst) return 0;
@@ -398,7 +399,7 @@ __device__ inline int big_solve(const BigPencil& p, double* smem, int maxit) {
       double *Hs = m.win, *Ts = Hs + nw * ld, *Us = Ts + nw * ld, *Vs = Us + nw * ld;
       big_load(p, kwtop, nw, Hs, Ts, Us, Vs, ld, ld);
       const double s = whole ? 0.0 : p.H[kwtop + (size_t)(kwtop - 1) * n];
-      if (tid < kRoleThreads) big_aed(nw, p.tol, s, whole ? 0 : 4);
+      if (tid < kRoleThreads) big_aed(nw, p.tol, s, whole ? 0 : nskip_table(n));
       __syncthreads();
       const int mu = sh->si[8], status = sh->si[9], changed = sh->si[10];
       if (status == 0 && changed) {
@@ -415,10 +416,8 @@ __device__ inline int big_solve(const BigPencil& p, double* smem, int maxit) {
       const int nd = status == 0 && changed ? nw - mu : 0;
       kbot -= nd;
       if (kbot < ktop) continue;
-      if (status == 0 && 100 * nd > 40 * nw) continue;  // nibble_table
-      int ns = nh >= 590 ? 64 : nh >= 150 ? nh / (int)lround(log2((double)nh)) : 10;  // ns_table
-      ns = max(2, ns - ns % 2);
-      ns = min(max(ns, 10), mu - (mu & 1));
+      if (status == 0 && 100 * nd > nibble_table(nh) * nw) continue;
+      const int ns = min(ns_table(nh), mu - (mu & 1));
       if (tid == 0) {
         int np = ns >= 2 ? big_pairs(sh->shift, sh->shift + kBigShifts, sh->shift + 2 * kBigShifts, mu, ns, sh->poly) : 0;
         if (stall > 0 && stall % 40 == 0) {

@@ -81,16 +81,16 @@ struct SolveStats {
 };
 
 // reference shift-count table (piparmq.f:504-533)
-inline int ns_table(int nh) {
+QZ_HD int ns_table(int nh) {
   int ns = 2;
   if (nh >= 30) ns = 4;
   if (nh >= 60) ns = 10;
-  if (nh >= 150) ns = std::max(10, (int)(nh / std::lround(std::log((double)nh) / std::log(2.0))));
+  if (nh >= 150) ns = nh / (int)lround(log((double)nh) / log(2.0));
   if (nh >= 590) ns = 64;
   if (nh >= 3000) ns = 128;
   if (nh >= 6000) ns = 256;
   if (nh >= 12000) ns = 512;
-  return std::max(2, ns - ns % 2);
+  return ns - ns % 2;
 }
 // Share of the window (in %) that an AED has to deflate for the next step to
 // be another AED instead of a sweep.  The reference's 14 up to nh = 6000
@@ -98,9 +98,9 @@ inline int ns_table(int nh) {
 // 0.6 (window 24) to 2 ms on one SM and a sweep 0.3 ms at n=200, 2.4 ms at
 // n=1800, so a sweep comes sooner.  Measured with 14 / 40 / 60: n=201 47 / 33 /
 // 38 ms, n=901 226 / 169 / 184, n=1800 482 / 410 / 439, n=4000 - / 1264 / 1328.
-inline int nibble_table(int nh) {
+QZ_HD int nibble_table(int nh) {
   if (nh <= 6000) return 40;
-  return std::min(100, (int)std::ceil(335.0 * std::pow((double)nh, -0.44)));
+  return (int)ceil(335.0 * pow((double)nh, -0.44));
 }
 
 // AED window of a pencil of order nh.  A window costs about nw^2 steps of one
@@ -109,7 +109,7 @@ inline int nibble_table(int nh) {
 // shrinks, costs 408 ms at n=1800 for 387.)  Measured (ms) with 24 / 32 / 48 / 56: n=201 24.8 / 29.5 / 32.6 / -,
 // n=500 75 / 75 / 96 / -, n=901 155 / 148 / 169 / -, n=1800 - / 497 / 387 /
 // 390, n=4000 - / - / 1264 / 1212.
-inline int nw_table(int nh) {
+QZ_HD int nw_table(int nh) {
   if (nh < 600) return 24;
   if (nh < 1200) return 32;
   if (nh < 3000) return 48;
@@ -124,7 +124,7 @@ inline int nw_table(int nh) {
 // 0.96, with 5 % infinite eigenvalues 1.10 / 0.99 / 1.04 / 1.02 / 0.98 / 1.00,
 // graded 1.03 / 1.03 / 1.01 / 1.02 / 0.99 / 0.98 (N(0,1) entries in T, where
 // much deflates early: 0.95 / 0.94 / 0.93 / 0.90 / 0.91 / 0.88).
-inline int nskip_table(int nh) { return nh >= 750 ? 0 : 4; }
+QZ_HD int nskip_table(int nh) { return nh >= 750 ? 0 : 4; }
 
 // Power of two applied to T before the iteration when T's magnitude is far
 // from H's (more than 2^30 apart), so that shift polynomials, whose
