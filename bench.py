@@ -741,6 +741,7 @@ def run_post(args, pkg):
     clk = clocks.stop()
     t = float(np.mean([x[0] for x in ts]))
     m, cnt = ts[-1][1], ts[-1][2]
+    launches = int(solver.stats()["launches"]) * args.steps
     te = []
     for _ in range(args.steps):
         Sh, Ph, Qh, Zh = (np.array(M, order="F") for M in (S, P, Q, Z))
@@ -773,7 +774,7 @@ def run_post(args, pkg):
                          "peak_source": "%s HBM copy bandwidth" % peak_kind,
                          "note": "factor-update bytes of the windows over the whole call; the swap chains "
                                  "inside each window are latency-bound on one CTA"},
-            "cpu_baseline": cpu, "clocks": clk, "gpu_launches": 3 * int(cnt[1]) + 2}
+            "cpu_baseline": cpu, "clocks": clk, "gpu_launches": launches}
     print(json.dumps(line), flush=True)
     solver.close()
 
@@ -820,6 +821,7 @@ def run_gghrd(args, pkg, solver, peaks, peak_kind, clocks):
     clocks.start()
     ts = [step() for _ in range(args.steps)]
     clk = clocks.stop()
+    launches = int(solver.stats()["launches"]) * args.steps
     t = float(np.mean(ts))
     # backward errors of the last reduction (FP64 products on the GPU)
     Hm, Tm, Qm, Zm, A0m, B0m = dA.T, dB.T, dQ.T, dZ.T, dA0.T, dB0.T
@@ -866,7 +868,7 @@ def run_gghrd(args, pkg, solver, peaks, peak_kind, clocks):
                          "peak_source": "%s HBM copy bandwidth" % peak_kind,
                          "note": "the walks' algorithmic bytes over the whole call; the bound is the chain "
                                  "of %d dependent rotation pairs on one SM (FP64 latency)" % pairs},
-            "cpu_baseline": cpu, "clocks": clk, "gpu_launches": windows + 2 * (n - 2) + 5}
+            "cpu_baseline": cpu, "clocks": clk, "gpu_launches": launches}
     print(json.dumps(line), flush=True)
 
 

@@ -1269,6 +1269,7 @@ int b200qz_tgsen_dev(b200qz_ctx* c, int ijob, int wantq, int wantz, const int* s
   qz::ReorderOut o;
   const cudaError_t e = qz::tgsen_device(c->stream, ijob, wantq != 0, wantz != 0, select, n, s, lds, t, ldt, q, ldq,
                                          z, ldz, alphar, alphai, beta, &o);
+  c->stats.launches = o.launches;
   if (e != cudaSuccess) return 10001;
   *m = o.m;
   *pl = o.pl;
@@ -1307,6 +1308,7 @@ int b200qz_tgsen_host(b200qz_ctx* c, int ijob, int wantq, int wantz, const int* 
   if (e == cudaSuccess)
     e = qz::tgsen_device(c->stream, ijob, wantq != 0, wantz != 0, select, n, ds, n, dt, n, dq, n, dz, n, de, de + n,
                          de + 2 * n, &o);
+  c->stats.launches = o.launches;
   if (e == cudaSuccess)
     e = cudaMemcpy2DAsync(s, (size_t)lds * sizeof(double), ds, w, w, n, cudaMemcpyDeviceToHost, c->stream);
   if (e == cudaSuccess)
@@ -1356,6 +1358,7 @@ static int gghrd_run(b200qz_ctx* c, int cq, int cz, bool qrows, int n, int ilo, 
   qz::GghrdOut o;
   const cudaError_t e =
       qz::gghrd_device(c->stream, cq, cz, qrows, n, ilo - 1, ihi - 1, a, lda, b, ldb, q, ldq, z, ldz, c->hr_win, &o);
+  c->stats.launches = o.launches;
   return e == cudaSuccess ? 0 : 10001;
 }
 

@@ -506,6 +506,8 @@ cudaError_t gghrd_device(cudaStream_t st, int icompq, int icompz, bool qrows, in
   if (icompq == 2) launch_identity(st, Q, ldq, n);
   if (icompz == 2) launch_identity(st, Z, ldz, n);
   if (n > 1) k_hr_zero_lower<<<std::min(1184, blocks_for(n * n)), kHrThreads, 0, st>>>(B, ldb, n);
+  int64_t launches = (icompq == 2) + (icompz == 2) + (n > 1), pairs = 0;
+  if (out) out->launches = launches;
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || n <= 1 || ihi - ilo < 2) return e;
   const int W = std::max(2, std::min(wmax, kHrMaxWin));
@@ -524,7 +526,6 @@ cudaError_t gghrd_device(cudaStream_t st, int icompq, int icompz, bool qrows, in
   e = cudaMemsetAsync(err, 0, sizeof(int), st);
   if (e != cudaSuccess) return e;
   HrArgs a{A, lda, B, ldb, Q, ldq, Z, ldz, rot, err, n, ihi, icompq != 0, icompz != 0, qrows};
-  int64_t launches = 0, pairs = 0;
   const int qz = hr_qz_warps(a);
   for (int jc = ilo; jc <= ihi - 2 && e == cudaSuccess; ++jc) {
     a.rot = rot + 4 * (size_t)n * ((jc - ilo) & 1);

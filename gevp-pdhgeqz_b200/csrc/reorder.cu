@@ -483,7 +483,7 @@ void add_job(UpdBatch& B, double* M, int64_t ld, int r0, int c0, int len, const 
 // sizes).
 cudaError_t dif_estimates(cudaStream_t st, const double* S, int64_t lds, const double* T, int64_t ldt, int m1,
                           int m2, const std::vector<int>& b1s, const std::vector<int>& b1z,
-                          const std::vector<int>& b2s, const std::vector<int>& b2z, double* dif) {
+                          const std::vector<int>& b2s, const std::vector<int>& b2z, double* dif, int64_t* launches) {
   const int n1 = (int)b1s.size(), n2 = (int)b2s.size();
   const size_t mn = (size_t)m1 * m2;
   DevMem mem;
@@ -519,6 +519,7 @@ cudaError_t dif_estimates(cudaStream_t st, const double* S, int64_t lds, const d
         return false;
       const int waves = g.na + g.nb - 1, width = g.na < g.nb ? g.na : g.nb;
       for (int d = 0; d < waves; ++d) k_sylv_gen_wave<<<(width + 7) / 8, 256, 0, st>>>(g, d);
+      *launches += waves;
       if (cudaGetLastError() != cudaSuccess) return false;
       if (cudaMemcpyAsync(x.data(), X, 2 * mn * sizeof(double), cudaMemcpyDeviceToHost, st) != cudaSuccess)
         return false;
@@ -593,6 +594,7 @@ cudaError_t tgsen_device(cudaStream_t st, int ijob, bool wantq, bool wantz, cons
       k_reorder_win<<<F.count, kReoThreads, reo_smem(wmax), st>>>(S, lds, T, ldt, dwin + F.first, dround, dswap, tol,
                                                                   U, V, status);
       k_reorder_status<<<1, 1, 0, st>>>(status);
+      out->launches += 2;
       // every left update of the phase before every right one
       for (int side = 0; side < 2; ++side) {
         UpdBatch B;
@@ -603,6 +605,7 @@ cudaError_t tgsen_device(cudaStream_t st, int ijob, bool wantq, bool wantz, cons
           const double* v = V + (size_t)i * kReoWin * kReoWin;
           if (B.njobs + 4 > kUpdMaxJobs) {
             launch_update(st, B, side);
+            ++out->launches;
             B.njobs = 0;
           }
           if (side == 0) {
@@ -615,7 +618,10 @@ cudaError_t tgsen_device(cudaStream_t st, int ijob, bool wantq, bool wantz, cons
             if (wantz) add_job(B, Z, ldz, 0, w.w0, n, v, w.wk);
           }
         }
-        if (B.njobs) launch_update(st, B, side);
+        if (B.njobs) {
+          launch_update(st, B, side);
+          ++out->launches;
+        }
       }
       e = cudaGetLastError();
       if (e != cudaSuccess) return e;
@@ -630,6 +636,7 @@ cudaError_t tgsen_device(cudaStream_t st, int ijob, bool wantq, bool wantz, cons
   }
   k_tgsen_signs<<<n, 256, 0, st>>>(S, lds, T, ldt, Q, ldq, n, wantq ? 1 : 0);
   k_tgsen_eigs<<<(n + 255) / 256, 256, 0, st>>>(S, lds, T, ldt, n, alphar, alphai, beta);
+  out->launches += 2;
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   if (out->info) {
@@ -678,6 +685,7 @@ cudaError_t tgsen_device(cudaStream_t st, int ijob, bool wantq, bool wantz, cons
     k_ssq_final<<<1, 32, 0, st>>>(part, kSsqBlocks, nrm);
     k_ssq_part<<<kSsqBlocks, 256, 0, st>>>(Lt, (int64_t)m1 * m2, part);
     k_ssq_final<<<1, 32, 0, st>>>(part, kSsqBlocks, nrm + 1);
+    out->launches += 2 + (nb1 + nb2 - 1) + 4;
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     double hn[2];
@@ -697,6 +705,7 @@ cudaError_t tgsen_device(cudaStream_t st, int ijob, bool wantq, bool wantz, cons
       double* part = (double*)nm.p;
       launch_sumsq(st, S, lds, 0, n, part + 592, part);
       launch_sumsq(st, T, ldt, 0, n, part + 593, part);
+      out->launches += 4;
       double hn[2];
       e = cudaMemcpyAsync(hn, part + 592, sizeof(hn), cudaMemcpyDeviceToHost, st);
       if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -708,7 +717,7 @@ cudaError_t tgsen_device(cudaStream_t st, int ijob, bool wantq, bool wantz, cons
         if (p < m1) { b1s.push_back(p); b1z.push_back(sz[k]); }
         else { b2s.push_back(p - m1); b2z.push_back(sz[k]); }
       }
-      e = dif_estimates(st, S, lds, T, ldt, m1, m2, b1s, b1z, b2s, b2z, out->dif);
+      e = dif_estimates(st, S, lds, T, ldt, m1, m2, b1s, b1z, b2s, b2z, out->dif, &out->launches);
       if (e != cudaSuccess) return e;
     }
   }

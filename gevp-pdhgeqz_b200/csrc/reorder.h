@@ -14,8 +14,9 @@ struct ReorderOut {
   double pr = 1.0;
   int info = 0;     // 1: a swap was rejected (the pencil is partly reordered)
   int swaps = 0;    // block swaps attempted
-  int windows = 0;  // window launches
+  int windows = 0;  // windows (a CTA each; a phase of them is one launch)
   double dif[2] = {0.0, 0.0};  // Difu, Difl estimates (ijob 3 and 5)
+  int64_t launches = 0;        // kernel launches
 };
 
 // select: host array of n flags.  S (lds), T (ldt), Q (ldq), Z (ldz) are

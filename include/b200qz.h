@@ -97,7 +97,8 @@ int b200qz_solve_host(b200qz_ctx* ctx, char job, char compq, char compz, int n, 
  * 16 chase updates, 17 infinite-eigenvalue deflation, 18 finalisation,
  * and inside the AED kernel 19 small QZ, 20 reordering, 21 spike
  * reflector + RQ update, 22 Hessenberg-triangular re-reduction;
- * 23 kernel launches issued by the solve, 24 AED windows whose small QZ
+ * 23 kernel launches issued by the solve (or by the last reduction or
+ * reordering, if that came after it), 24 AED windows whose small QZ
  * did not converge (they deflate nothing and supply diagonal shifts),
  * 25 sweeps run with exceptional shifts (after 40 iterations without
  * deflation), 26 rows left unconverged, 27/28 active block where an
