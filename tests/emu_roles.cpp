@@ -1,8 +1,11 @@
-// The window QZ with a role per warp (qz_roles.cuh), run as a thread block on
-// the host (warp_emu.h).  roles_host.inc is that header with its flag loads,
-// flag stores and predicated stores, which are PTX, left out: they are below.
+// The window QZ and the early deflation with a role per warp (qz_roles.cuh),
+// and the chase (qz_chase_roles.cuh), run as thread blocks on the host
+// (warp_emu.h).  roles_host.inc and chase_host.inc are those headers with
+// their flag loads, flag stores, predicated stores and named barrier, which
+// are PTX, left out: they are below.
 #include "warp_emu.h"
 
+#include <algorithm>
 #include <cfloat>
 
 #include "qz_window.cuh"
@@ -37,8 +40,12 @@ inline void role_post(bool on, int* p, int v) {
 }
 inline double role_rsqrt(double x) { return 1.0 / sqrt(x); }
 inline double role_rcp(double x) { return 1.0 / x; }
+inline void chase_bar();
 }  // namespace qz
-#include "roles_host.inc"
+#include "chase_host.inc"
+namespace qz {
+inline void chase_bar() { emu::named_barrier(1, kChaseMain); }
+}  // namespace qz
 
 using namespace qz;
 
@@ -100,6 +107,89 @@ int emu_role_qz(int n, double* H, double* T, double* Q, double* Z, unsigned slow
       Z[i + j * n] = m[3 * n * ld + i + j * ld];
     }
   return status;
+}
+
+// Early deflation of a window (n x n, in place) with spike entry s (k_aed_win);
+// out3: undeflated, status, changed; shifts: 3 n.
+void emu_aed(int n, double* H, double* T, double* Q, double* Z, double s, int nskip, double* shifts, int* out3,
+             unsigned slow) {
+  kRoleSpin = 1 << 22;
+  const int ld = n % 2 == 0 ? n + 1 : n;
+  std::vector<double> mem((size_t)4 * n * ld + kRoleDoubles + 64 + 4 * n + 8, 0.0);
+  double* const m = mem.data();
+  std::vector<int> si(64);
+  for (int j = 0; j < n; ++j)
+    for (int i = 0; i < n; ++i) {
+      m[i + j * ld] = H[i + j * n];
+      m[n * ld + i + j * ld] = T[i + j * n];
+      m[2 * n * ld + i + j * ld] = m[3 * n * ld + i + j * ld] = i == j ? 1.0 : 0.0;
+    }
+  RoleBuf* const rb = (RoleBuf*)(m + 4 * n * ld);
+  emu::run(kRoleThreads, slow, (char*)m, [&](int tid) {
+    EmuExec x{tid, kRoleThreads, si.data(), (double*)rb + kRoleDoubles};
+    WinState w;
+    w.n = n;
+    w.H = MatV{m, ld};
+    w.T = MatV{m + n * ld, ld};
+    w.Q = MatV{m + 2 * n * ld, ld};
+    w.Z = MatV{m + 3 * n * ld, ld};
+    w.wantq = w.wantz = true;
+    w.tol.safmin = DBL_MIN;
+    w.tol.ulp = DBL_EPSILON;
+    w.tol.smlnum = DBL_MIN * ((double)n / DBL_EPSILON);
+    w.tol.htol = w.tol.ttol = DBL_EPSILON * n;
+    const int qz = cta_role_qz(x, w, 30 * n, rb);
+    if (qz == 0) cta_std_all(x, w, x.sd + 64);
+    cta_aed_deflate(
+        x, w, s, shifts, shifts + n, shifts + 2 * n, qz, [&]() { return cta_role_spike(x, w, s, nskip, false, rb); },
+        [&](int mm) { return cta_role_hessred(x, w, mm, rb); });
+  });
+  for (int k = 0; k < 3; ++k) out3[k] = si[8 + k];
+  for (int j = 0; j < n; ++j)
+    for (int i = 0; i < n; ++i) {
+      H[i + j * n] = m[i + j * ld];
+      T[i + j * n] = m[n * ld + i + j * ld];
+      Q[i + j * n] = m[2 * n * ld + i + j * ld];
+      Z[i + j * n] = m[3 * n * ld + i + j * ld];
+    }
+}
+
+// Chase of nb bulges (polynomials coef, 3 each) through a window that ends its
+// block: introduced at the top, pushed off at the bottom (k_chase_win).
+// Returns 0, or 1 if a wait gave up.
+int emu_chase(int n, double* H, double* T, double* U, double* V, const double* coef, int nb, unsigned slow) {
+  kRoleSpin = 1 << 22;
+  const int ld = n % 2 == 0 ? n + 1 : n;
+  const size_t ring = 4 * (size_t)n * ld;
+  std::vector<double> mem(ring + chase_ring_doubles(nb) + 8, 0.0);
+  double* const m = mem.data();
+  std::vector<Bulge> bl(nb);
+  ChaseShare share{};
+  int tmax = 0;
+  for (int k = 0; k < nb; ++k) {
+    bl[k] = Bulge{-3 * k, 3 * k, n - 1 + 3 * k, 1, coef[3 * k], coef[3 * k + 1], coef[3 * k + 2]};
+    tmax = std::max(tmax, bl[k].thi);
+  }
+  for (int j = 0; j < n; ++j)
+    for (int i = 0; i < n; ++i) {
+      m[i + j * ld] = H[i + j * n];
+      m[n * ld + i + j * ld] = T[i + j * n];
+      m[2 * n * ld + i + j * ld] = m[3 * n * ld + i + j * ld] = i == j ? 1.0 : 0.0;
+    }
+  bool ok = false;
+  emu::run(kChaseRoleThreads, slow, (char*)m, [&](int tid) {
+    const bool r = cta_chase_roles(n, n - 1, MatV{m, ld}, MatV{m + n * ld, ld}, MatV{m + 2 * n * ld, ld},
+                                   MatV{m + 3 * n * ld, ld}, bl.data(), nb, tmax, m + ring, &share);
+    if (tid == 0) ok = r;
+  });
+  for (int j = 0; j < n; ++j)
+    for (int i = 0; i < n; ++i) {
+      H[i + j * n] = m[i + j * ld];
+      T[i + j * n] = m[n * ld + i + j * ld];
+      U[i + j * n] = m[2 * n * ld + i + j * ld];
+      V[i + j * n] = m[3 * n * ld + i + j * ld];
+    }
+  return ok ? 0 : 1;
 }
 
 // role_wait_done by warp 0 while warps 1 and 2 post their counts up to v:

@@ -25,6 +25,7 @@ struct Fiber {
   std::vector<char> stack;
   bool done = false;
   bool waiting = false;  // at a rendezvous
+  int bar = 0;           // the named barrier, if it is one
   uint64_t slot = 0;     // its contribution to a collective
 };
 struct Warp {
@@ -39,7 +40,7 @@ struct Block {
   std::vector<Fiber> f;
   std::vector<Warp> w;
   ucontext_t home;
-  int cur = 0, barrier = 0;
+  int cur = 0, barrier = 0, named[16] = {};
   unsigned slow = 0;  // warps that run only when the others are stuck
   std::function<void(int)> body;
   char* arena = nullptr;  // "shared memory" (base of 32-bit addresses)
@@ -86,6 +87,24 @@ inline void block_barrier() {
   if (++b.barrier == total) {
     b.barrier = 0;
     for (Fiber& x : b.f) x.waiting = false;
+    return;
+  }
+  while (b.f[me].waiting) yield();
+}
+// a barrier of `count` of the threads (bar.sync id, count)
+inline void named_barrier(int id, int count) {
+  Block& b = *block();
+  const int me = b.cur;
+  b.f[me].waiting = true;
+  b.f[me].bar = id;
+  b.w[me / kLanes].spins = 0;
+  if (++b.named[id] == count) {
+    b.named[id] = 0;
+    for (Fiber& x : b.f)
+      if (x.waiting && x.bar == id) {
+        x.waiting = false;
+        x.bar = 0;
+      }
     return;
   }
   while (b.f[me].waiting) yield();
@@ -176,7 +195,11 @@ inline void run(int threads, unsigned slow, char* arena, const std::function<voi
 struct double2 {
   double x, y;
 };
+struct int2 {
+  int x, y;
+};
 inline double2 make_double2(double x, double y) { return double2{x, y}; }
+inline int2 make_int2(int x, int y) { return int2{x, y}; }
 inline uint64_t emu_bits(double v) {
   uint64_t u;
   memcpy(&u, &v, 8);
@@ -187,6 +210,13 @@ inline double emu_double(uint64_t u) {
   memcpy(&v, &u, 8);
   return v;
 }
+struct EmuThreadIndex {
+  struct X {
+    operator int() const { return emu::block()->cur; }
+  } x;
+};
+static const EmuThreadIndex threadIdx{};
+inline void __syncthreads() { emu::block_barrier(); }
 inline void __syncwarp() {
   emu::meet(0);
   emu::Block& b = *emu::block();
