@@ -16,9 +16,11 @@
 // from the bottom up, on the window's diagonal block of B and the column's
 // entries of A; the row rotations come from the column of A alone.  The rest
 // of a window's rotations is applied with the next window (or after the
-// column's last) as walks.  This file has the pieces one thread can run
-// (hr_g_chain, cta_hr_zchain and the walks, by which the form is checked on
-// the host); hessred.cu has the device's split of them.  The walks:
+// column's last) as walks.  This file has the rotation, the operands and the
+// pieces of a sequential form on one host thread (hr_g_chain, cta_hr_zchain
+// and the walks), against which the windowed form was first checked;
+// hessred.cu has the device's split of them, of which it takes the rotation,
+// hr_g_chain for entries out of range, and the operands.  The walks:
 //   (a) its Z on the rows of B the next window's block holds (CTA 0),
 //   (e) its Z on the rows of B above those,
 //   (f) its G on the columns of B right of the window,

@@ -96,8 +96,14 @@ QZ_HD int ns_table(int nh) {
 // be another AED instead of a sweep.  The reference's 14 up to nh = 6000
 // (piparmq.f:495-496) weighs an AED against its own sweeps; here an AED costs
 // 0.6 (window 24) to 2 ms on one SM and a sweep 0.3 ms at n=200, 2.4 ms at
-// n=1800, so a sweep comes sooner.  Measured with 14 / 40 / 60: n=201 47 / 33 /
-// 38 ms, n=901 226 / 169 / 184, n=1800 482 / 410 / 439, n=4000 - / 1264 / 1328.
+// n=1800, so a sweep comes sooner.  Measured with 14 / 20 / 28 / 40 (ms): forms
+// of dense pairs n=901 182 / 174 / 167 / 159, n=1800 474 / 447 / 411 / 391,
+// n=4000 1395 / 1282 / 1229 / 1174, graded n=2000 539 / 504 / 479 / 454 (60 at
+// n=1800: 439 for 410, with earlier kernels).  Above 3000 it depends on the
+// pencil: with 14 there and 40 below, forms of dense pairs take 1.03 times as
+// long at n=4000 and 5000 and 1.01 at 9000, graded ones the same, while with
+// N(0,1) entries in T, where AEDs go on deflating, n=4000 takes 0.92, n=5000
+// 0.76 and the graded pencil of order 10000 0.78.
 QZ_HD int nibble_table(int nh) {
   if (nh <= 6000) return 40;
   return (int)ceil(335.0 * pow((double)nh, -0.44));

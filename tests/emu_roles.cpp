@@ -2,44 +2,13 @@
 // and the chase (qz_chase_roles.cuh), run as thread blocks on the host
 // (warp_emu.h).  roles_host.inc and chase_host.inc are those headers with
 // their flag loads, flag stores, predicated stores and named barrier, which
-// are PTX, left out: they are below.
-#include "warp_emu.h"
-
+// are PTX, left out: they are in emu_prims.h and below.
 #include <algorithm>
 #include <cfloat>
 
-#include "qz_window.cuh"
+#include "emu_prims.h"
+
 namespace qz {
-inline int role_ld(const int* p) { return emu::polled(p); }
-inline void role_st(int* p, int v) {
-  *(volatile int*)p = v;
-  emu::posted();
-}
-inline unsigned role_sm(const void* p) { return (unsigned)((const char*)p - emu::block()->arena); }
-inline double* emu_at(unsigned a) { return (double*)(emu::block()->arena + a); }
-inline void role_put(bool on, unsigned a, double v) {
-  if (on) *emu_at(a) = v;
-}
-inline void role_put3(bool on, unsigned a, unsigned st, double v0, double v1, double v2) {
-  if (!on) return;
-  *emu_at(a) = v0;
-  *emu_at(a + st) = v1;
-  *emu_at(a + 2 * st) = v2;
-}
-inline void role_put8(bool on, unsigned a, double v0, double v1, double v2, double v3, double v4, double v5, double v6,
-                      double v7) {
-  const double v[8] = {v0, v1, v2, v3, v4, v5, v6, v7};
-  if (on) memcpy(emu_at(a), v, sizeof v);
-}
-inline void role_put_int2(bool on, unsigned a, int v0, int v1) {
-  const int v[2] = {v0, v1};
-  if (on) memcpy(emu_at(a), v, sizeof v);
-}
-inline void role_post(bool on, int* p, int v) {
-  if (on) role_st(p, v);
-}
-inline double role_rsqrt(double x) { return 1.0 / sqrt(x); }
-inline double role_rcp(double x) { return 1.0 / x; }
 inline void chase_bar();
 }  // namespace qz
 #include "chase_host.inc"

@@ -18,9 +18,9 @@ _pd = ctypes.POINTER(ctypes.c_double)
 RIGHT, Q, Z = 0x06, 0x28, 0xC0  # warps of the right transformations, of Q and of Z
 
 
-def _build(out):
-    """Host build of qz_roles.cuh and qz_chase_roles.cuh without their PTX; the
-    polls after which a wait gives up are a variable."""
+def _host_headers(out):
+    """qz_roles.cuh and qz_chase_roles.cuh for the host: without their PTX, the
+    polls after which a wait gives up a variable."""
     with open(os.path.join(CSRC, "qz_roles.cuh")) as f:
         text = f.read()
     a = text.index("__device__ __forceinline__ int role_ld")
@@ -38,6 +38,10 @@ def _build(out):
     text = text.replace(bar[0], "").replace("#ifdef __CUDACC__", "#if 1").replace("qz_roles.cuh", "roles_host.inc")
     with open(os.path.join(out, "chase_host.inc"), "w") as f:
         f.write(text)
+
+
+def _build(out):
+    _host_headers(out)
     lib = os.path.join(out, "libemu.so")
     subprocess.run(["g++", "-O2", "-ffp-contract=off", "-shared", "-fPIC", "-std=c++17", "-Wno-unknown-pragmas",
                     "-I", out, "-I", CSRC, "-I", HERE, os.path.join(HERE, "emu_roles.cpp"), "-o", lib],

@@ -22,7 +22,6 @@ namespace emu {
 constexpr int kLanes = 32;
 struct Fiber {
   ucontext_t ctx;
-  std::vector<char> stack;
   bool done = false;
   bool waiting = false;  // at a rendezvous
   int bar = 0;           // the named barrier, if it is one
@@ -137,6 +136,14 @@ inline void entry(unsigned lo, unsigned hi) {
   for (;;) yield();
 }
 
+// the fibers' stacks, kept from block to block
+constexpr size_t kStack = 256 << 10;
+inline char* stack(int i) {
+  static std::vector<char*> pool;
+  while ((int)pool.size() <= i) pool.push_back((char*)malloc(kStack));
+  return pool[i];
+}
+
 // one turn of a warp: every lane that can run, until all have met or polled;
 // true if some lane was not just waiting
 inline bool turn(Block& b, int warp) {
@@ -161,13 +168,13 @@ inline void run(int threads, unsigned slow, char* arena, const std::function<voi
   b.body = body;
   b.arena = arena;
   block() = &b;
-  for (Fiber& x : b.f) {
-    x.stack.resize(256 << 10);
-    getcontext(&x.ctx);
-    x.ctx.uc_stack.ss_sp = x.stack.data();
-    x.ctx.uc_stack.ss_size = x.stack.size();
-    x.ctx.uc_link = nullptr;
-    makecontext(&x.ctx, (void (*)())entry, 2, (unsigned)(uintptr_t)&b, (unsigned)((uintptr_t)&b >> 32));
+  for (int i = 0; i < threads; ++i) {
+    ucontext_t& c = b.f[i].ctx;
+    getcontext(&c);
+    c.uc_stack.ss_sp = stack(i);
+    c.uc_stack.ss_size = kStack;
+    c.uc_link = nullptr;
+    makecontext(&c, (void (*)())entry, 2, (unsigned)(uintptr_t)&b, (unsigned)((uintptr_t)&b >> 32));
   }
   const int warps = (int)b.w.size();
   constexpr long kStuck = 8 * kLanes;  // polls in a row after which a warp counts as stuck
@@ -216,6 +223,21 @@ struct EmuThreadIndex {
   } x;
 };
 static const EmuThreadIndex threadIdx{};
+struct EmuIndex {
+  int x = 0;
+};
+inline EmuIndex& emu_block_index() {
+  static EmuIndex i;
+  return i;
+}
+inline EmuIndex& emu_grid_size() {
+  static EmuIndex i;
+  return i;
+}
+inline EmuIndex& emu_block_size() {
+  static EmuIndex i;
+  return i;
+}
 inline void __syncthreads() { emu::block_barrier(); }
 inline void __syncwarp() {
   emu::meet(0);
@@ -245,3 +267,10 @@ inline double __shfl_up_sync(unsigned, double v, int d) {
 inline double __shfl_xor_sync(unsigned, double v, int d) { return emu_double(emu::meet(emu_bits(v))[emu::lane_id() ^ d]); }
 inline int __ffs(unsigned v) { return __builtin_ffs((int)v); }
 inline int __double2hiint(double v) { return (int)(emu_bits(v) >> 32); }
+inline int __double2loint(double v) { return (int)emu_bits(v); }
+inline double __hiloint2double(int hi, int lo) { return emu_double((uint64_t)(uint32_t)hi << 32 | (uint32_t)lo); }
+inline int atomicExch(int* p, int v) {
+  const int old = *p;
+  *p = v;
+  return old;
+}
