@@ -493,11 +493,8 @@ __device__ inline void role_follow(WinState& w, RoleBuf* rb, int warp, int lane)
         break;
       }
     }
-    if (!__any_sync(0xffffffffu, go)) {
-      // the end, unless the wait gave up: steps would be lost then
-      if (lane == 0 && (role_ld(&rb->stop) == 0 || role_ld(&rb->ready) > g)) role_st(&rb->err, 1);
-      return;
-    }
+    // the end, or the wait gave up: cta_role_qz compares the counts
+    if (!__any_sync(0xffffffffu, go)) return;
     __syncwarp();
     const double* sl = rb->ring[g & (kRoleRing - 1)];
     const int s = ((const int*)(sl + 8))[0];
@@ -616,9 +613,13 @@ __device__ int cta_role_qz(X& x, WinState& w, int maxit, RoleBuf* rb) {
     }
     x.sync();
     const int code = rb->code, f = rb->arg[0], jz = rb->arg[1], il = rb->arg[2], err = rb->err;
+    // a follower that gave up has not done every step; the core waits for the
+    // Q and Z warps only when the ring is full, so it may not have noticed
+    bool lost = false;
+    for (int i = 0; i < 8; ++i)
+      if ((kRoleAll >> i) & 1) lost = lost || rb->done[i] != rb->ready;
     x.sync();
-    // (a follower may give up when the core is past its last row)
-    if (err != 0 || code == 2) return il >= 0 ? il + 1 : 1;
+    if (err != 0 || code == 2 || lost) return il >= 0 ? il + 1 : 1;
     if (code == 0) return 0;
     // a zero on T's diagonal: infinite eigenvalue, all threads
     if (jz == f) {

@@ -101,7 +101,7 @@ QZ_HD int ns_table(int nh) {
 // n=4000 1395 / 1282 / 1229 / 1174, graded n=2000 539 / 504 / 479 / 454 (60 at
 // n=1800: 439 for 410, with earlier kernels).  Above 3000 it depends on the
 // pencil: with 14 there and 40 below, forms of dense pairs take 1.03 times as
-// long at n=4000 and 5000 and 1.01 at 9000, graded ones the same, while with
+// long at n=4000, 1.04 at 5000 and 1.01 at 9000, graded ones too, while with
 // N(0,1) entries in T, where AEDs go on deflating, n=4000 takes 0.92, n=5000
 // 0.76 and the graded pencil of order 10000 0.78.
 QZ_HD int nibble_table(int nh) {
