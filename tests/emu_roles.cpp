@@ -36,9 +36,9 @@ extern "C" {
 int emu_role_qz(int n, double* H, double* T, double* Q, double* Z, unsigned slow, int spin) {
   kRoleSpin = spin;
   const int ld = n % 2 == 0 ? n + 1 : n;
-  std::vector<double> mem((size_t)4 * n * ld + kRoleDoubles + 3 * n + 8, 0.0);
+  std::vector<double> mem((size_t)4 * n * ld + kRoleDoubles + 3 * n + 8, NAN);  // (as uninitialised)
   double* const m = mem.data();
-  std::vector<int> si(64);
+  std::vector<int> si(64, -1);
   double hs = 0.0, ts = 0.0;
   for (int j = 0; j < n; ++j)
     for (int i = 0; i < n; ++i) {
@@ -84,9 +84,9 @@ void emu_aed(int n, double* H, double* T, double* Q, double* Z, double s, int ns
              unsigned slow) {
   kRoleSpin = 1 << 22;
   const int ld = n % 2 == 0 ? n + 1 : n;
-  std::vector<double> mem((size_t)4 * n * ld + kRoleDoubles + 64 + 4 * n + 8, 0.0);
+  std::vector<double> mem((size_t)4 * n * ld + kRoleDoubles + 64 + 4 * n + 8, NAN);
   double* const m = mem.data();
-  std::vector<int> si(64);
+  std::vector<int> si(64, -1);
   for (int j = 0; j < n; ++j)
     for (int i = 0; i < n; ++i) {
       m[i + j * ld] = H[i + j * n];
@@ -130,7 +130,7 @@ int emu_chase(int n, double* H, double* T, double* U, double* V, const double* c
   kRoleSpin = 1 << 22;
   const int ld = n % 2 == 0 ? n + 1 : n;
   const size_t ring = 4 * (size_t)n * ld;
-  std::vector<double> mem(ring + chase_ring_doubles(nb) + 8, 0.0);
+  std::vector<double> mem(ring + chase_ring_doubles(nb) + 8, NAN);
   double* const m = mem.data();
   std::vector<Bulge> bl(nb);
   ChaseShare share{};

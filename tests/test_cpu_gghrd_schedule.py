@@ -43,7 +43,7 @@ def emu(tmp_path_factory):
     with open(os.path.join(out, "cuda_runtime.h"), "w") as f:
         f.write("#pragma once\n")
     lib = os.path.join(out, "libemuhr.so")
-    subprocess.run(["g++", "-O2", "-ffp-contract=off", "-shared", "-fPIC", "-std=c++17", "-Wno-unknown-pragmas",
+    subprocess.run(["g++", "-O2", "-U_FORTIFY_SOURCE", "-ffp-contract=off", "-shared", "-fPIC", "-std=c++17", "-Wno-unknown-pragmas",
                     "-I", out, "-I", CSRC, "-I", HERE, os.path.join(HERE, "emu_hessred.cpp"), "-o", lib],
                    check=True, capture_output=True, timeout=300)
     L = ctypes.CDLL(lib)

@@ -43,7 +43,7 @@ def _host_headers(out):
 def _build(out):
     _host_headers(out)
     lib = os.path.join(out, "libemu.so")
-    subprocess.run(["g++", "-O2", "-ffp-contract=off", "-shared", "-fPIC", "-std=c++17", "-Wno-unknown-pragmas",
+    subprocess.run(["g++", "-O2", "-U_FORTIFY_SOURCE", "-ffp-contract=off", "-shared", "-fPIC", "-std=c++17", "-Wno-unknown-pragmas",
                     "-I", out, "-I", CSRC, "-I", HERE, os.path.join(HERE, "emu_roles.cpp"), "-o", lib],
                    check=True, capture_output=True, timeout=300)
     L = ctypes.CDLL(lib)
@@ -82,7 +82,7 @@ def _run(L, H, T, slow, spin=1 << 22):
 
 
 @pytest.mark.parametrize("n,kind,seed", [(9, "dense", 1), (20, "dense", 2), (20, "split", 3), (24, "zero_t", 4),
-                                         (34, "split", 5)])
+                                         (34, "split", 5), (34, "dense", 6), (66, "split", 7)])
 def test_any_order_of_the_warps(emu, lapack, n, kind, seed):
     H, T = _pencil(n, kind, seed)
     rc, first = _run(emu, H, T, 0)

@@ -6,6 +6,7 @@
 // warp in turn, or chosen warps only when no other can get on.  Code that
 // waits for what it reads gives the same bits under any order.
 #pragma once
+#include <setjmp.h>
 #include <ucontext.h>
 
 #include <cmath>
@@ -21,7 +22,9 @@ namespace emu {
 
 constexpr int kLanes = 32;
 struct Fiber {
-  ucontext_t ctx;
+  ucontext_t ctx;        // where it begins
+  jmp_buf at;            // where it goes on
+  bool begun = false;
   bool done = false;
   bool waiting = false;  // at a rendezvous
   int bar = 0;           // the named barrier, if it is one
@@ -38,7 +41,7 @@ struct Warp {
 struct Block {
   std::vector<Fiber> f;
   std::vector<Warp> w;
-  ucontext_t home;
+  jmp_buf home;
   int cur = 0, barrier = 0, named[16] = {};
   unsigned slow = 0;  // warps that run only when the others are stuck
   std::function<void(int)> body;
@@ -53,9 +56,17 @@ inline Block*& block() {
   static Block* b = nullptr;
   return b;
 }
-inline void yield() {
+// (jumps between stacks; contexts are for the first entry alone, as they save
+// the signal mask by a system call)
+__attribute__((noinline)) inline void yield() {
   Block& b = *block();
-  swapcontext(&b.f[b.cur].ctx, &b.home);
+  if (_setjmp(b.f[b.cur].at) == 0) _longjmp(b.home, 1);
+}
+__attribute__((noinline)) inline void enter(Block& b, Fiber& x) {
+  if (_setjmp(b.home) != 0) return;
+  if (x.begun) _longjmp(x.at, 1);
+  x.begun = true;
+  setcontext(&x.ctx);
 }
 inline int lane_id() { return block()->cur % kLanes; }
 
@@ -153,7 +164,7 @@ inline bool turn(Block& b, int warp) {
     if (x.done || x.waiting) continue;
     ran = true;
     b.cur = warp * kLanes + l;
-    swapcontext(&b.home, &x.ctx);
+    enter(b, x);
   }
   return ran;
 }
